@@ -324,7 +324,7 @@ def gpu_arm(args):
     es = 8 if dtype == "f64" else 4
     alg_bytes = 2 * C * es * v * args.time_steps
     value = sum_over_ranks(alg_bytes / sec64 / 1e9, world)
-    kernel64 = plan64.module.gen.step_kernels[plan64.last_tile][0]
+    kernel64 = plan64.module.gen.kernels[plan64.last_tile][0]
     tb64 = codegen.tile_steps(plan64.last_tile)
 
     if args.device_only or args.time_steps != N_STEPS:
@@ -344,7 +344,7 @@ def gpu_arm(args):
     f32_final = plan32.unpack(traj32[-1], 1)
     f64_final = plan64.unpack(traj64[-1], 1)
     f32_err = float(torch.linalg.norm(f32_final - f64_final) / torch.linalg.norm(f64_final))
-    kernel32 = plan32.module.gen.step_kernels[plan32.last_tile][0]
+    kernel32 = plan32.module.gen.kernels[plan32.last_tile][0]
     tb32 = codegen.tile_steps(plan32.last_tile)
     del traj32, traj64, f32_final, f64_final
     torch.cuda.empty_cache()

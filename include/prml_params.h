@@ -77,11 +77,12 @@ typedef struct prml_step_params {
    * and ny columns per plane as above, nz planes (1 for 0/1/2-D), planes
    * nx * pitch elements apart; a 3D kernel's tile depth and TMA box depth */
   int nz;
-  int tile_z;
+  int tile_z;              /* 2D marching kernels: rows per job (see edge_rows) */
   int box_planes;
   double inv_2dx2, inv_dxx2, two_dx2;
   float inv_2dx2_f, inv_dxx2_f, two_dx2_f;
-  int pad3;
+  int jobs_per_cta;        /* tiles one CTA takes at once (marching kernels:
+                              one per warp); 0 or 1 otherwise            */
   const double* coord2;
   const float* coord2_f;
   /* dx^2 per kernel axis (2D: axes 0, 1; 3D: the planes' axis in dxx2):
@@ -98,7 +99,9 @@ typedef struct prml_step_params {
    * and nothing else happens (2: the multi-round kernel waits for one
    * grid-barrier arrival more than the grid has).  0 in every solve. */
   int wait_probe;
-  int pad4;
+  /* 2D marching kernels: rows per job of the first and last strip of
+   * columns, tile_z of the strips between */
+  int edge_rows;
   /* Per-instance offset (in half-step tables) added to bc_slot0, or NULL:
    * a batch whose instances start at different times of one set of
    * time-dependent boundary tables (Parareal slices). */

@@ -321,7 +321,7 @@ class StepParams(ctypes.Structure):
         ("inv_2dx2_f", ctypes.c_float),
         ("inv_dxx2_f", ctypes.c_float),
         ("two_dx2_f", ctypes.c_float),
-        ("pad3", _c_int),
+        ("jobs_per_cta", _c_int),
         ("coord2", _p),
         ("coord2_f", _p),
         ("dxx0", _c_d),
@@ -329,7 +329,7 @@ class StepParams(ctypes.Structure):
         ("dxx2", _c_d),
         ("wait_limit_ns", ctypes.c_ulonglong),
         ("wait_probe", _c_int),
-        ("pad4", _c_int),
+        ("edge_rows", _c_int),
         ("bc_inst_slot", _p),
     ]
 

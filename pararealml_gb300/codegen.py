@@ -62,6 +62,19 @@ TB_CONFIGS: Tuple[Tuple[int, int, int, int], ...] = tuple(
 # (rows per thread R, warps per CTA); the tile is 4 R rows by 8 warps x 16
 # bytes of columns, keyed (4 R, cols, threads, 1, 0, "w")
 WALK_CONFIGS: Tuple[Tuple[int, int], ...] = ((1, 4), (2, 2), (2, 4), (4, 2), (4, 4))
+# marching kernels (march_body) on 2D meshes: (columns per lane, pipeline
+# depth) per element size; a job is a chunk of rows of one strip of columns,
+# sized at each launch so that there are MARCH_JOBS[k] jobs per SM (march_rows).
+# Multi-stage steps have one stage per pipeline level, single-stage
+# steps one time step.
+MARCH_MULTI: Dict[int, Tuple[int, ...]] = {4: (2, 4), 8: (1, 2)}
+MARCH_SINGLE: Dict[int, Tuple[Tuple[int, int], ...]] = {4: ((4, 2), (4, 4)), 8: ((2, 1), (2, 2))}
+MARCH_JOBS: Tuple[int, ...] = (4, 8, 12, 16, 20, 24)
+# cost of a row of a strip on a column face over one between (esize -> ratio):
+# 64 x 257^2 RK4 diffusion in float32 2.58 / 2.41 / 2.66 / 2.93 ms at 1 / 1.5 /
+# 2 / 2.5, 16 x 257^2 in float64 9.1 / 10.1 / 11.4 / 11.7 ms
+MARCH_EDGE = {4: 1.5, 8: 1.0}
+MARCH_THREADS = 128
 # 3D tiles (rows, cols, threads, 1, planes)
 TILE_CONFIGS_3D: Tuple[Tuple[int, int, int, int, int], ...] = (
     (8, 32, 256, 1, 2),
@@ -640,8 +653,27 @@ def _rhs_function(name: str, rows: Sequence[int], low: LoweredProblem, fast: boo
     return "\n".join(lines) + "\n"
 
 
+def _side_columns(low: LoweredProblem) -> Tuple[int, bool]:
+    """(mask of the components some derivative of which is read, whether a
+    mixed second derivative is): which side columns of a window the
+    marching kernels fetch from the neighbouring lanes."""
+    mask, corners = 0, False
+    for expr in low.rhs:
+        for s in expr.free_symbols:
+            prefix, idx = _parse(s)
+            if prefix in ("t", "x", "y"):
+                continue
+            if prefix in ("y-gradient", "y-hessian", "y-laplacian"):
+                mask |= 1 << idx[0]
+                corners = corners or (prefix == "y-hessian" and idx[1] != idx[2])
+            else:  # divergence and curl name several components
+                mask |= (1 << low.n_comp) - 1
+    return mask, corners
+
+
 _TEMPLATE_FILES = (
     ("csrc", "fdm_step.cuh"),
+    ("csrc", "fdm_march.cuh"),
     ("csrc", "fdm_step3d.cuh"),
     ("include", "prml_params.h"),
 )
@@ -682,6 +714,45 @@ def is_walk(tile) -> bool:
     return len(tile) > 5 and tile[5] == "w"
 
 
+def is_march(tile) -> bool:
+    """Whether a tile key names a marching kernel (march_body)."""
+    return len(tile) > 5 and tile[5] == "m"
+
+
+def march_tile(jobs: int, vw: int, depth: int, steps: int = 1) -> tuple:
+    """Tile key of a marching kernel: ``jobs`` jobs (warps) per SM, ``vw``
+    columns per lane, pipeline ``depth`` (halo lanes on both sides), ``steps``
+    time steps per launch."""
+    cols = 32 * vw - 2 * (-(-depth // vw)) * vw
+    return (jobs, cols, MARCH_THREADS, steps, 0, "m", vw)
+
+
+def march_rows(tile, nx: int, ny: int, batch: int, esize: int, sms: int) -> Tuple[int, int]:
+    """Rows per job of a marching kernel, (strips between, first and last
+    strip): the fewest rows for which the launch has at most ``tile[0]`` jobs
+    per SM, so that all warps run at once and end together.  Measured on
+    64 x 257^2 RK4 diffusion in float32: 2.4 ms per 100 steps with jobs that
+    fill the resident warps once, 2.7 ms with twice as many, 3.9 ms with fixed
+    chunks of 32 rows.  A job's fixed cost is about 1.5 rows per pipeline level (rows
+    computed before its first output row); a strip on a column face costs
+    MARCH_EDGE times as much per row, so its chunks are shorter (float64, where
+    the float64 pipe is the bound, pays nothing extra there)."""
+    strips = -(-ny // tile[1])
+    edges = min(2, strips)
+    inner = strips - edges
+    fixed = 1.5 * ((32 * tile[6] - tile[1]) // 2)
+    jobs = max(tile[0] * sms, batch * strips)
+    weight = MARCH_EDGE[esize]
+    cost = fixed + 1.0
+    while True:
+        rows = min(nx, max(1, int(cost - fixed)))
+        edge = min(nx, max(1, int(cost / weight - fixed)))
+        if batch * (inner * -(-nx // rows) + edges * -(-nx // edge)) <= jobs:
+            # even chunks: the same number of jobs, no short last one
+            return -(-nx // -(-nx // rows)), -(-nx // -(-nx // edge))
+        cost += 1.0
+
+
 def walk_tile(rows_per_thread: int, warps: int, esize: int) -> tuple:
     """Tile key of the register-window kernel with R rows per thread and
     ``warps`` warps per CTA."""
@@ -689,6 +760,8 @@ def walk_tile(rows_per_thread: int, warps: int, esize: int) -> tuple:
 
 
 def kernel_name(kind: str, dtype: str, tile) -> str:
+    if is_march(tile):
+        return f"prml_march_{dtype}_v{tile[6]}" + (f"_k{tile[3]}" if tile[3] > 1 else "")
     if is_walk(tile):
         return f"prml_walk_{dtype}_{tile[0]}x{tile[1]}x{tile[2]}"
     if tile_planes(tile):
@@ -755,10 +828,19 @@ class GeneratedModule:
     rhs_kernel: Tuple[str, int, Tuple[int, int, int]]
     n_comp: int = 1
     multi_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
+    # marching kernels: tile (jobs per SM, cols, threads, steps, 0, "m", columns per lane) -> (name, smem)
+    march_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
+
+    @property
+    def kernels(self) -> Dict[tuple, Tuple[str, int]]:
+        """Every step kernel: tile -> (name, dynamic shared memory)."""
+        return {**self.step_kernels, **self.march_kernels}
 
     def box(self, tile, mode: int = 0) -> Tuple[int, int]:
         """TMA box (rows, cols) a kernel of this module stages."""
         esize = 8 if self.dtype == "f64" else 4
+        if is_march(tile):  # no tile is staged: any box the tensor map accepts
+            return 1, 16 // esize
         return region(tile, halo(self.integrator, self.invariant, mode, tile), esize)
 
     def box_planes(self, tile) -> int:
@@ -807,7 +889,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
     if three_d and comp:
         raise NotImplementedError("compensated float32 is not available on 3D meshes")
     body = [
-        '#include "fdm_step3d.cuh"' if three_d else '#include "fdm_step.cuh"',
+        '#include "fdm_step3d.cuh"' if three_d else '#include "fdm_step.cuh"\n#include "fdm_march.cuh"',
         "",
         "struct Eq {",
         f"  static constexpr int C = {low.n_comp};",
@@ -818,6 +900,12 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         f"  static constexpr bool EXACT_DIV = {'true' if exact_div else 'false'};",
         f"  static constexpr bool FAST = {'true' if fast else 'false'};",
         f"  static constexpr bool EQUAL_DX = {'true' if low.dx_k[0] == low.dx_k[1] else 'false'};",
+        f"  static constexpr unsigned HMASK = {_side_columns(low)[0]}u;",
+        f"  static constexpr bool CORNERS = {'true' if _side_columns(low)[1] else 'false'};",
+        f"  static constexpr bool DYNAMIC = {'true' if low.dynamic else 'false'};",
+        # column-face values may be read once per row: static conditions, no
+        # mixed derivative, and no lane that touches both column faces
+        f"  static constexpr bool PRE = {'true' if not low.dynamic and not _side_columns(low)[1] and low.ny > 8 else 'false'};",
         f"  static constexpr unsigned long long NEU_MASK = {low.neu_mask}ull;",
         f"  static constexpr unsigned long long DIR_MASK = {low.dir_mask}ull;",
         f"  static __device__ constexpr int dcomp(int i) {{ return {_chain(d_rows)}; }}",
@@ -888,6 +976,26 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
             )
     if not step_kernels:
         raise NotImplementedError("no tile configuration fits in shared memory")
+    # marching kernels: 2D meshes, no Jacobi solve between steps, no
+    # compensated state; multi-stage systems of dy/dt rows only (an LHS.Y
+    # row's value belongs to the step's start, several rows behind the end of
+    # the pipeline).  Modules of implicit integrators take no steps.
+    march_kernels = {}
+    if low.x_dimension == 2 and not low.lap_idx and not comp and not exact_div and (single_stage or not y_rows):
+        shapes = MARCH_SINGLE[esize] if single_stage else tuple((vw, integrator) for vw in MARCH_MULTI[esize])
+        for vw, depth in shapes:
+            # windows and slopes of wider systems do not fit in registers
+            if not single_stage and (3 * depth + 1) * low.n_comp * vw * esize // 4 > 110:
+                continue
+            steps = depth if single_stage else 1
+            tiles = [march_tile(rows, vw, depth, steps) for rows in MARCH_JOBS]
+            name = kernel_name("march", dtype, tiles[0])
+            march_kernels.update({tile: (name, 0) for tile in tiles})
+            body.append(
+                f'extern "C" __global__ void __launch_bounds__({MARCH_THREADS}, 3) {name}'
+                f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin) "
+                f"{{ (void)tin; prml::march_body<{ctype}, Eq, {integrator}, {vw}, {depth}, {MARCH_THREADS}>(p); }}"
+            )
     rtile = (16, 32, 128)
     rname = kernel_name("rhs", dtype, rtile)
     rsm = smem_bytes(low, integrator, invariant, rtile, esize, 1)
@@ -922,4 +1030,5 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         rhs_kernel=(rname, rsm, rtile),
         n_comp=low.n_comp,
         multi_kernels=multi_kernels,
+        march_kernels=march_kernels,
     )

@@ -250,9 +250,10 @@ int prml_module_kernel(void* module, const char* name, int smem_bytes, void** ke
     return fail(PRML_ERR_ARG, std::string("kernel ") + name + " not found: " + cu_name(r));
   }
   k->smem = smem_bytes;
-  /* the step kernels stage everything in shared memory and gain nothing
-   * from L1: ask for the largest shared-memory carveout (a preference) */
-  g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_PREFERRED_SHARED_MEMORY_CARVEOUT, 100);
+  /* the staged step kernels keep everything in shared memory and gain
+   * nothing from L1: ask for the largest shared-memory carveout (a
+   * preference); kernels without dynamic shared memory for the largest L1 */
+  g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_PREFERRED_SHARED_MEMORY_CARVEOUT, smem_bytes > 0 ? 100 : 0);
   /* opt in to the requested dynamic size whatever it is: a kernel with
    * static shared memory too (the multi-round kernels' group tables) can
    * exceed the 48 KB default with less than 48 KB of dynamic memory */
@@ -378,11 +379,22 @@ static int persistent_grid(Kernel* k, int block, const prml_step_params* base, i
   }
   const int tz = base->tile_z > 0 ? base->tile_z : 1;
   const int nz = base->nz > 0 ? base->nz : 1;
-  const long long tiles = (long long)((base->ny + tile_y - 1) / tile_y) *
-                          ((base->nx + tile_x - 1) / tile_x) * ((nz + tz - 1) / tz) * base->batch;
+  long long tiles = (long long)((base->ny + tile_y - 1) / tile_y) *
+                    ((base->nx + tile_x - 1) / tile_x) * ((nz + tz - 1) / tz) * base->batch;
+  if (tiles + k->grid_cap >= (1LL << 31)) return fail(PRML_ERR_ARG, "too many tiles for one launch (2^31)");
+  if (base->jobs_per_cta > 1) {
+    /* marching kernels: one job per warp, the first and last strip of columns
+     * in chunks of edge_rows rows, the strips between in chunks of tile_z */
+    if (base->edge_rows < 1) return fail(PRML_ERR_ARG, "marching kernels need edge_rows");
+    const long long strips = (base->ny + tile_y - 1) / tile_y, edges = strips < 2 ? strips : 2;
+    const long long jobs = base->batch * (edges * ((base->nx + base->edge_rows - 1) / base->edge_rows) +
+                                          (strips - edges) * ((base->nx + tz - 1) / tz));
+    if (jobs + (long long)k->grid_cap * base->jobs_per_cta >= (1LL << 31))
+      return fail(PRML_ERR_ARG, "too many tiles for one launch (2^31)");
+    tiles = (jobs + base->jobs_per_cta - 1) / base->jobs_per_cta;
+  }
   long long cap = k->grid_cap;
   if (base->max_ctas > 0 && base->max_ctas < cap) cap = base->max_ctas;
-  if (tiles + cap >= (1LL << 31)) return fail(PRML_ERR_ARG, "too many tiles for one launch (2^31)");
   /* as many rounds of tiles as the resident CTAs need, and the tiles spread
    * evenly over them: no CTA walks more tiles than another plus one */
   const long long rounds = (tiles + cap - 1) / cap;

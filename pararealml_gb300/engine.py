@@ -248,9 +248,10 @@ class StencilPlan:
         self._tuned: Dict[bool, Tuple[int, ...]] = {}  # trajectory pattern -> tuned tile
         self._tuned_ctas: Dict[bool, int] = {}  # trajectory pattern -> tuned grid cap (0 = fill the GPU)
         self._user_ctas = 0
+        self._march_rows: Dict[tuple, Tuple[int, int]] = {}
         self.last_tile: Optional[Tuple[int, ...]] = self.tile
         self.last_ctas = 0  # grid cap of the latest run (0 = every resident CTA)
-        if self.tile is not None and self.tile not in self.module.gen.step_kernels:
+        if self.tile is not None and self.tile not in self.module.gen.kernels:
             raise ValueError(f"tile {self.tile} is not instantiated for this module")
 
     # ------------------------------------------------------------------
@@ -736,7 +737,7 @@ class StencilPlan:
             cur = out
 
     def _step_kernel(self, tile):
-        name, smem = self.module.gen.step_kernels[tile]
+        name, smem = self.module.gen.kernels[tile]
         return self.module.kernel(name, smem)
 
     def run(
@@ -900,17 +901,22 @@ class StencilPlan:
 
     def _launch(self, tile, y0, y0_bstride, traj, traj_bstride, traj_step_stride, wa, wb,
                 n_steps, save_every, t0, dt) -> None:
-        if codegen.is_walk(tile):
-            # the register-window kernels move 16 bytes per access: every
-            # buffer, instance and step must start on a 16-byte boundary
+        if codegen.is_walk(tile) or codegen.is_march(tile):
+            # these kernels move up to 16 bytes per access: every buffer,
+            # instance and step must start on a 16-byte boundary
             vw = 16 // self.esize
             strides = (y0_bstride, traj_bstride, traj_step_stride, self.inst)
             addrs = [a for a in (y0, traj, wa, wb) if a]
             if any(a % 16 for a in addrs) or any(s % vw for s in strides):
-                raise ValueError("register-window step kernels need 16-byte aligned states and strides")
+                raise ValueError("register-window and marching step kernels need 16-byte aligned states and strides")
         rows, cols = self.module.gen.box(tile)
         self.params.tb_max = codegen.tile_steps(tile)
-        self.params.tile_z = max(1, codegen.tile_planes(tile))
+        if codegen.is_march(tile):
+            self.params.tile_z, self.params.edge_rows = self.march_rows(tile, self.params.batch)
+            self.params.jobs_per_cta = tile[2] // 32
+        else:
+            self.params.tile_z = max(1, codegen.tile_planes(tile))
+            self.params.jobs_per_cta = 1
         self.params.box_planes = self.module.gen.box_depth(tile)
         _native.check(
             _native.lib().prml_fdm_run(
@@ -921,12 +927,29 @@ class StencilPlan:
             "fdm run",
         )
 
+    def march_rows(self, tile, batch: int) -> Tuple[int, int]:
+        """Rows per job of a marching kernel for ``batch`` instances
+        (``codegen.march_rows``)."""
+        key = (tile, batch)
+        rows = self._march_rows.get(key)
+        if rows is None:
+            if len(self._march_rows) > 256:
+                self._march_rows.clear()
+            rows = self._march_rows[key] = codegen.march_rows(tile, self.rows, self.ny, batch, self.esize, self._sms())
+        return rows
+
+    def _sms(self) -> int:
+        import torch
+
+        return torch.cuda.get_device_properties(self.device).multi_processor_count
+
     def rhs(self, y, f, t: float) -> None:
         """Right-hand side of every equation at (t, y) into ``f`` (device states)."""
         name, smem, tile = self.module.gen.rhs_kernel
         k = self.module.kernel(name, smem)
         rows, cols = self.module.gen.box(tile, mode=1)
         self.params.tile_z = max(1, codegen.tile_planes(tile))
+        self.params.jobs_per_cta = 1
         self.params.box_planes = self.module.gen.box_depth(tile, mode=1)
         _native.check(
             _native.lib().prml_fdm_rhs(
@@ -984,14 +1007,14 @@ class StencilPlan:
             return self._tuned[full]
         key = f"{self.module.gen.key}:{self.nz}x{self.rows}x{self.ny}:b{self.batch}:{'full' if full else 'final'}:v3"
         cached = _tune_cache_load().get(key)
-        if isinstance(cached, dict) and tuple(cached.get("tile", ())) in self.module.gen.step_kernels:
+        if isinstance(cached, dict) and tuple(cached.get("tile", ())) in self.module.gen.kernels:
             self._tuned[full] = tuple(cached["tile"])
             self._tuned_ctas[full] = int(cached.get("ctas", 0))
             return self._tuned[full]
         import torch as _torch
 
         sms = _torch.cuda.get_device_properties(self.device).multi_processor_count
-        cands = list(self.module.gen.step_kernels)
+        cands = list(self.module.gen.step_kernels) + list(getattr(self.module.gen, "march_kernels", {}))
         reps = 16  # a multiple of every temporal block; best of 3 rounds per tile
         # timing launches read boundary table 0 only: a time-dependent run's
         # tables may cover fewer half steps than the timing launches take
@@ -1011,7 +1034,8 @@ class StencilPlan:
                 # grid density: every resident CTA (one round of tiles), or
                 # fewer CTAs per SM that each walk several tiles and stage the
                 # next tile while computing the current one
-                caps = [0] + [sms * c for c in (2, 4, 8) if c < occ.value]
+                # (marching jobs are sized by their rows instead)
+                caps = [0] + [sms * c for c in (2, 4, 8) if c < occ.value and not codegen.is_march(tile)]
 
                 def go(n, tile=tile):
                     self._launch(
