@@ -20,7 +20,8 @@
  * `while diff > tol`, so a NaN change also stops it).  Divisions by the
  * step sizes and denominators are products with host-computed reciprocals.
  *
- * One cooperative launch per solve: the CTAs of an instance split its
+ * Instances of up to 32768 values run on one thread-block cluster each
+ * (jacobi_cluster).  Larger ones in one cooperative launch per solve: the CTAs of an instance split its
  * (component, vertex) items, two ping-pong buffers hold the estimates, and
  * one grid barrier per iteration separates the iterations.  Every CTA sums
  * the per-CTA partial norms in the same order, so all CTAs take the same
@@ -30,6 +31,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <string>
 
 #include "prml_internal.h"
@@ -818,6 +820,416 @@ bool staged_shape(const prml_jacobi_params& p, int sms, Stage<T>& sg, int& G, in
   return false;
 }
 
+/* Cluster kernel: one thread-block cluster per instance, for solves whose
+ * estimates fit in the registers and shared memory of one cluster.  The
+ * vertices (dense index, every solved component) are split evenly over the
+ * cluster's CTAs; a thread keeps its VT vertices' estimate and right-hand side
+ * in registers, each CTA two copies of its estimates plus a halo of one mesh
+ * stride on both sides in shared memory.  An iteration reads the neighbours
+ * from shared memory and writes the new estimates there and, with remote
+ * stores counted on an mbarrier, into the two neighbouring CTAs' halos: a CTA
+ * waits for its two neighbours only, nothing is computed twice and nothing
+ * leaves the SMs.  On Cartesian meshes the denominator and the ghosts' constant
+ * parts are folded into the weights and the right-hand side.
+ * Every CK iterations the squared changes are summed in a fixed order, every
+ * CTA receives every other's sums and all take the same decision; a block that
+ * contains the stop iteration is repeated from its start (kept in registers)
+ * up to it.  No CTA waits on another cluster, so any batch runs.
+ *
+ * Why: the staged kernel pays a grid barrier through L2 per block and
+ * recomputes its band's halo rows (7 rows for 4 owned at 101 x 81 in float64,
+ * where the float64 pipe issues two operations per clock and SM).  At 101 x 81
+ * an iteration takes 1.35 us in float64 (6.4 us staged) and 0.49 us in float32
+ * (2.8 us).  What is left in float64 is the pipe: 512 vertices x 6 operations
+ * per SM are 0.8 us; in float32 the halo store, the neighbour's wait and the CTA
+ * barrier.  A cluster barrier per iteration instead of the halo mbarriers took
+ * 3.0 / 1.8 us, face vertices on their own branch 2.4 / 1.5 us. */
+constexpr int CT = 512;  // threads per CTA
+constexpr int CK = 16;   // iterations between two stop tests
+constexpr int CL_MAX = 16;
+
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+/* address of `p` (own shared memory) in CTA `rank` of the cluster */
+__device__ __forceinline__ unsigned remote_addr(const void* p, unsigned rank) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void st_remote(unsigned a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+/* remote store that counts its bytes on the receiving CTA's mbarrier */
+__device__ __forceinline__ void st_async(unsigned a, float v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(a), "f"(v), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned a, double v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(a), "d"(v), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool halo_landed(const unsigned long long* bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+/* Split of V vertices over CL CTAs: counts differ by at most one. */
+struct Split {
+  int CL, base, rem, H; /* H: halo = the longest stride of the mesh */
+  __host__ __device__ int count(int r) const { return base + (r < rem ? 1 : 0); }
+  __host__ __device__ int first(int r) const { return r * base + (r < rem ? r : rem); }
+  __host__ __device__ int most() const { return base + (rem ? 1 : 0); }
+  __host__ __device__ int line() const { return most() + 2 * H; } /* elements of one buffer */
+};
+
+template <typename T, int CS, int D, int VT>
+__global__ void __launch_bounds__(CT) jacobi_cluster(const prml_jacobi_params p, T* __restrict__ state,
+                                                     const double* __restrict__ y_init, unsigned char* scratch,
+                                                     Layout L, Div d12, Div d2, Split sp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double cpart[CK][CL_MAX]; /* [iteration][CTA] squared changes of the block */
+  __shared__ unsigned long long bar[2]; /* halo of copy 0 / 1 has arrived */
+  __shared__ int hit_s, dead;
+  const int n_lap = p.n_lap;
+  const T* coef = static_cast<const T*>(p.coef);
+  unsigned* status = reinterpret_cast<unsigned*>(scratch + L.control + 128);
+  Geo<T> g;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    g.n[a] = p.n[a];
+    g.inv_dxx[a] = T(p.inv_dxx[a]);
+    g.two_dx[a] = T(p.two_dx[a]);
+  }
+  g.V = g.n[0] * g.n[1] * g.n[2];
+  g.stride[2] = 1;
+  g.stride[1] = g.n[2];
+  g.stride[0] = g.n[1] * g.n[2];
+  g.d12 = d12;
+  g.d2 = d2;
+  g.dir = static_cast<const T*>(p.dirichlet);
+  g.neu = static_cast<const T*>(p.neumann);
+  g.dmask = p.dir_mask;
+  g.nmask = p.neu_mask;
+  g.comps = p.comps;
+  g.flen = p.face_len;
+  g.fbase = p.face_base;
+  g.pitch = p.pitch;
+  g.cstride = p.cstride;
+
+  const int rank = (int)cluster_rank();
+  const int b = blockIdx.x / sp.CL;
+  const int cnt = sp.count(rank), v0 = sp.first(rank), H = sp.H, line = sp.line();
+  T* const buf = reinterpret_cast<T*>(smem_raw); /* two copies of [n_lap][line] */
+  const int zero = n_lap * line, copy = (n_lap * line + 4) / 4 * 4; /* one element stays zero: the halo outside the mesh */
+  T* sqs = buf + 2 * copy;                       /* [CK][CT] */
+  T* st = state + (long long)b * p.inst;
+
+  /* this thread's vertices: item e = (component l, offset o of the CTA's) */
+  int off[VT], vtx[VT], crd[VT][3], lc[VT];
+  /* Cartesian meshes: where the two neighbours along each axis are (outside
+   * the mesh: the mirrored vertex of a Neumann ghost, or the zero element) */
+  int nb[VT][D][2];
+  bool fixed[VT];
+  constexpr unsigned NONE = 0xffffffffu;
+  unsigned to_prev[VT], to_next[VT]; /* halo slots in the neighbours' first copy */
+  const unsigned bar_prev = rank > 0 ? remote_addr(bar, rank - 1) : NONE;
+  const unsigned bar_next = rank + 1 < sp.CL ? remote_addr(bar, rank + 1) : NONE;
+  const unsigned halo_bytes = (unsigned)((int)(rank > 0) + (int)(rank + 1 < sp.CL)) * (unsigned)(H * n_lap * (int)sizeof(T));
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < 2; ++q)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(bar + q)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    dead = 0;
+  }
+  bool have[VT], in[VT];
+  T y[VT], lap[VT], start[VT];
+  T weight[3] = {T(0), T(0), T(0)};
+  if constexpr (CS == 0) {
+#pragma unroll
+    for (int ka = 3 - D; ka < 3; ++ka) weight[ka] = g.inv_dxx[ka] * coef[0];
+  }
+#pragma unroll
+  for (int t = 0; t < VT; ++t) {
+    const int e = threadIdx.x + t * CT;
+    have[t] = e < cnt * n_lap;
+    to_prev[t] = to_next[t] = NONE;
+    if (!have[t]) continue;
+    const int l = e / cnt;
+    int o = e - l * cnt;
+    /* the vertices that the neighbours wait for come first */
+    if (cnt >= 2 * H && o >= H) o = o < 2 * H ? cnt - 2 * H + o : o - H;
+    int z, i, j;
+    vtx[t] = v0 + o;
+    decode<D>(vtx[t], d12, d2, z, i, j);
+    crd[t][0] = z;
+    crd[t][1] = i;
+    crd[t][2] = j;
+    off[t] = l * line + H + o;
+    lc[t] = p.lap_comp[l];
+    in[t] = j > 0 && j < g.n[2] - 1;
+    if (D >= 2) in[t] = in[t] && i > 0 && i < g.n[1] - 1;
+    if (D == 3) in[t] = in[t] && z > 0 && z < g.n[0] - 1;
+    lap[t] = st[lc[t] * g.cstride + ((long long)z * g.n[1] + i) * g.pitch + j];
+    y[t] = constrain<T, D>(g, T(y_init[((long long)b * g.V + vtx[t]) * n_lap + l]), lc[t], z, i, j);
+    fixed[t] = false;
+    if constexpr (CS == 0) {
+      /* the right-hand side times the denominator, the constant part of any
+       * Neumann ghost folded in */
+      fixed[t] = !in[t] && constrain<T, D>(g, T(0), lc[t], z, i, j) == constrain<T, D>(g, T(1), lc[t], z, i, j);
+      T r = -lap[t] * coef[0];
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        const int ka = 3 - D + a, q = crd[t][ka], sd = g.stride[ka];
+        nb[t][a][0] = off[t] - sd;
+        nb[t][a][1] = off[t] + sd;
+        T gv;
+        if (q == 0) {
+          const bool ghost = table_value(g, g.neu, g.nmask, 2 * ka, lc[t], z, i, j, gv);
+          nb[t][a][0] = ghost ? off[t] + sd : zero;
+          if (ghost) r = fma_(-g.two_dx[ka] * gv, weight[ka], r);
+        }
+        if (q == g.n[ka] - 1) {
+          const bool ghost = table_value(g, g.neu, g.nmask, 2 * ka + 1, lc[t], z, i, j, gv);
+          nb[t][a][1] = ghost ? off[t] - sd : zero;
+          if (ghost) r = fma_(g.two_dx[ka] * gv, weight[ka], r);
+        }
+      }
+      lap[t] = r;
+    }
+    if (o < H && rank > 0) to_prev[t] = remote_addr(buf + l * line + H + sp.count(rank - 1) + o, rank - 1);
+    if (o >= cnt - H && rank + 1 < sp.CL) to_next[t] = remote_addr(buf + l * line + o - (cnt - H), rank + 1);
+  }
+  if (threadIdx.x < 2) buf[threadIdx.x * copy + zero] = T(0);
+  unsigned phase[2] = {0u, 0u};
+  /* own estimates into copy w and the neighbours' halos; returns when the
+   * CTA's copy and halo are complete.  A neighbour can only be one iteration
+   * ahead, and only after every vertex here that reads its halo has been
+   * sent, so two copies suffice.  The wait is bounded: on expiry the status
+   * is set, no later wait is entered, and a NaN norm ends every CTA's loop. */
+  auto publish = [&](int w) {
+    const unsigned shift = (unsigned)(w * copy * (int)sizeof(T));
+    if (threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(bar + w)), "r"(halo_bytes)
+                   : "memory");
+#pragma unroll
+    for (int t = 0; t < VT; ++t) {
+      if (!have[t]) continue;
+      buf[w * copy + off[t]] = y[t];
+      if (to_prev[t] != NONE) st_async(to_prev[t] + shift, y[t], bar_prev + 8u * (unsigned)w);
+      if (to_next[t] != NONE) st_async(to_next[t] + shift, y[t], bar_next + 8u * (unsigned)w);
+    }
+    __syncthreads();
+    const unsigned parity = (w ? phase[1] : phase[0]) & 1u;
+    if (w) ++phase[1];
+    else ++phase[0];
+    if (!halo_landed(bar + w, parity) && !*(volatile int*)&dead) {
+      const unsigned long long t0 = global_ns();
+      while (!halo_landed(bar + w, parity)) {
+        if (global_ns() - t0 > BARRIER_NS) {
+          atomicOr(status, 2u);
+          *(volatile int*)&dead = 1;
+          break;
+        }
+      }
+    }
+  };
+  /* one iteration from copy w into the other; the thread's squared change */
+  auto iterate = [&](int w) {
+    T sq = T(0);
+#pragma unroll
+    for (int t = 0; t < VT; ++t) {
+      if (!have[t]) continue;
+      T r;
+      if constexpr (CS == 0) {
+        /* one add and one multiply-add per axis, the denominator folded into
+         * the weights and the right-hand side; faces take the same path, so
+         * no warp diverges */
+        const T* cw = buf + w * copy;
+        r = lap[t];
+#pragma unroll
+        for (int a = D - 1; a >= 0; --a) r = fma_(add_(cw[nb[t][a][0]], cw[nb[t][a][1]]), weight[3 - D + a], r);
+        r = fixed[t] ? y[t] : r;
+      } else {
+        const T* cl = buf + w * copy + off[t] - vtx[t]; /* cl[v]: estimate of dense vertex v */
+        if (in[t]) {
+          r = estimate<T, CS, D, false, true>(g, cl, coef, lap[t], lc[t], crd[t][0], crd[t][1], crd[t][2], vtx[t]);
+        } else {
+          r = estimate<T, CS, D, true, true>(g, cl, coef, lap[t], lc[t], crd[t][0], crd[t][1], crd[t][2], vtx[t]);
+          r = constrain<T, D>(g, r, lc[t], crd[t][0], crd[t][1], crd[t][2]);
+        }
+      }
+      const T d = r - y[t];
+      sq = fma_(d, d, sq);
+      y[t] = r;
+    }
+    publish(w ^ 1);
+    return sq;
+  };
+
+  cluster_sync(); /* every CTA of the cluster runs, its barriers set, before its memory is written */
+  publish(0);
+  int w = 0;
+  long long it0 = 0;
+  int result = -1; /* 0: no iteration, 1: stopped after it0, -1: not converged */
+  if (!(__longlong_as_double(0x7ff0000000000000LL) > p.tol)) {
+    result = 0; /* tol = inf: the constrained initial estimate */
+  } else {
+    for (;;) {
+      const long long left = p.max_iterations - it0;
+      const int Kb = (int)(left < CK ? left : CK);
+      const int w0 = w;
+#pragma unroll
+      for (int t = 0; t < VT; ++t) start[t] = y[t];
+      for (int s = 0; s < Kb; ++s) {
+        sqs[s * CT + threadIdx.x] = iterate(w);
+        w ^= 1;
+      }
+      /* CTA sums: 32 threads per iteration add 16 values each, then a
+       * shuffle tree */
+      {
+        __syncthreads();
+        const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        T a = T(0);
+        if (s < Kb) {
+#pragma unroll
+          for (int q = 0; q < CT / 32; ++q) a += sqs[s * CT + q * 32 + lane];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+          if (lane < sp.CL)
+            st_remote(remote_addr(&cpart[s][rank], lane), dead ? __longlong_as_double(0x7ff8000000000000LL) : double(a));
+        }
+      }
+      cluster_sync();
+      if (threadIdx.x < 32) {
+        bool stop = false;
+        if ((int)threadIdx.x < Kb) {
+          double t = 0.0;
+          for (int r = 0; r < sp.CL; ++r) t += cpart[threadIdx.x][r];
+          stop = !(sqrt(t) > p.tol);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, stop);
+        if (threadIdx.x == 0) hit_s = m ? __ffs(m) - 1 : -1;
+      }
+      __syncthreads();
+      const int hit = hit_s; /* the same in every CTA; cpart is next written after a cluster barrier */
+      if (hit >= 0) {
+        it0 += hit + 1;
+        result = 1;
+        if (hit + 1 < Kb) { /* repeat the block up to the stop iteration */
+#pragma unroll
+          for (int t = 0; t < VT; ++t) y[t] = start[t];
+          publish(w0);
+          w = w0;
+          for (int s = 0; s <= hit; ++s) {
+            iterate(w);
+            w ^= 1;
+          }
+        }
+        break;
+      }
+      it0 += Kb;
+      if (it0 >= p.max_iterations) break;
+    }
+  }
+  if (rank == 0 && threadIdx.x == 0)
+    reinterpret_cast<long long*>(scratch + L.iters)[b] = result == 0 ? 0 : (result > 0 ? it0 : -1);
+#pragma unroll
+  for (int t = 0; t < VT; ++t)
+    if (have[t])
+      st[lc[t] * g.cstride + ((long long)crd[t][0] * g.n[1] + crd[t][1]) * g.pitch + crd[t][2]] = y[t];
+  cluster_sync(); /* no CTA leaves while another may still write to it */
+}
+
+/* Launch shape of the cluster kernel: the largest cluster the GPU takes (16
+ * CTAs, else 8, ..) that leaves every CTA at least one halo's worth of
+ * vertices, at most 4 items per thread.  False: the instance is too large. */
+template <typename T>
+bool cluster_shape(const prml_jacobi_params& p, int max_cluster, Split& sp, int& vt, int& smem) {
+  const int d = 3 - p.first_axis;
+  const long long V = (long long)p.n[0] * p.n[1] * p.n[2];
+  const long long H = d == 3 ? (long long)p.n[1] * p.n[2] : (d == 2 ? p.n[2] : 1);
+  if (V > (1 << 20)) return false;
+  int CL = max_cluster;
+  while (CL > 1 && V / CL < H) CL >>= 1;
+  if (V / CL < H) return false;
+  sp.CL = CL;
+  sp.base = (int)(V / CL);
+  sp.rem = (int)(V - (long long)sp.base * CL);
+  sp.H = (int)H;
+  const long long items = (long long)sp.most() * p.n_lap;
+  if (items > 4 * CT) return false;
+  vt = items <= CT ? 1 : (items <= 2 * CT ? 2 : 4);
+  smem = (int)sizeof(T) * (2 * ((p.n_lap * sp.line() + 4) / 4 * 4) + CK * CT);
+  return smem <= STAGED_SMEM_MAX;
+}
+
+template <typename T, int CS, int D, int VT>
+cudaError_t launch_cluster(const prml_jacobi_params& p, T* st, const double* y_init, unsigned char* sc, const Layout& L,
+                           Div d12, Div d2, const Split& sp, int smem, cudaStream_t s) {
+  auto kern = jacobi_cluster<T, CS, D, VT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess && sp.CL > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(sp.CL * p.batch));
+  cfg.blockDim = dim3(CT);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)sp.CL;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, p, st, y_init, sc, L, d12, d2, sp);
+}
+
+/* Largest cluster (16, 8, ..) of the kernel that device `dev` can hold, asked
+ * once per device (with the most shared memory a launch may take). */
+template <typename T, int CS, int D>
+int max_cluster(int dev) {
+  static std::atomic<int> known[64];
+  if (dev >= 0 && dev < 64 && known[dev].load() > 0) return known[dev].load();
+  const int smem = STAGED_SMEM_MAX;
+  auto kern = jacobi_cluster<T, CS, D, 4>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  for (int CL = CL_MAX; CL > 1; CL >>= 1) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)CL);
+    cfg.blockDim = dim3(CT);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)CL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) {
+      if (dev >= 0 && dev < 64) known[dev].store(CL);
+      return CL;
+    }
+  }
+  cudaGetLastError();
+  return 1;
+}
+
 template <typename T, int CS, int D>
 int launch(const prml_jacobi_params& p, void* state, const double* y_init, void* scratch, long long scratch_bytes,
            long long* iterations, cudaStream_t s) {
@@ -829,9 +1241,22 @@ int launch(const prml_jacobi_params& p, void* state, const double* y_init, void*
   const long long V = (long long)p.n[0] * p.n[1] * p.n[2];
   Stage<T> sg{};
   int G = 0, smem = 0;
-  const bool staged = staged_shape<T, CS, D>(p, sms, sg, G, smem);
-  const void* kern;
-  if (staged) {
+  Div d12 = make_div(p.n[1] * p.n[2]), d2 = make_div(p.n[2]);
+  T* st = static_cast<T*>(state);
+  unsigned char* sc = static_cast<unsigned char*>(scratch);
+  /* one cluster per instance where it fits */
+  Split sp{};
+  int vt = 0;
+  bool clustered = cluster_shape<T>(p, CL_MAX, sp, vt, smem);
+  if (clustered) {
+    const int most = max_cluster<T, CS, D>(dev);
+    if (most < sp.CL) clustered = cluster_shape<T>(p, most, sp, vt, smem);
+  }
+  const bool staged = !clustered && staged_shape<T, CS, D>(p, sms, sg, G, smem);
+  const void* kern = nullptr;
+  if (clustered) {
+    G = 1;
+  } else if (staged) {
     kern = (const void*)jacobi_staged<T, CS, D>;
   } else {
     int occ = 0;
@@ -850,14 +1275,16 @@ int launch(const prml_jacobi_params& p, void* state, const double* y_init, void*
   if (scratch_bytes < L.total) return prml_set_error(PRML_ERR_ARG, "prml_anti_laplacian: scratch too small");
   cudaError_t e = cudaMemsetAsync(scratch, 0, 256, s);
   if (e != cudaSuccess) return prml_set_error(PRML_ERR_CUDA, std::string("prml_anti_laplacian: ") + cudaGetErrorString(e));
-  T* st = static_cast<T*>(state);
-  unsigned char* sc = static_cast<unsigned char*>(scratch);
   prml_jacobi_params pc = p;
   Layout Lc = L;
-  Div d12 = make_div(p.n[1] * p.n[2]), d2 = make_div(p.n[2]);
   void* args_direct[] = {&pc, &st, (void*)&y_init, &sc, &Lc, &G, &d12, &d2};
   void* args_staged[] = {&pc, &st, (void*)&y_init, &sc, &Lc, &G, &d12, &d2, &sg};
-  e = cudaLaunchCooperativeKernel(kern, dim3((unsigned)(G * p.batch)), dim3(staged ? JS : JT), staged ? args_staged : args_direct,
+  if (clustered)
+    e = vt == 1 ? launch_cluster<T, CS, D, 1>(p, st, y_init, sc, L, d12, d2, sp, smem, s)
+                : (vt == 2 ? launch_cluster<T, CS, D, 2>(p, st, y_init, sc, L, d12, d2, sp, smem, s)
+                           : launch_cluster<T, CS, D, 4>(p, st, y_init, sc, L, d12, d2, sp, smem, s));
+  else
+    e = cudaLaunchCooperativeKernel(kern, dim3((unsigned)(G * p.batch)), dim3(staged ? JS : JT), staged ? args_staged : args_direct,
                                   staged ? (size_t)smem : 0, s);
   if (e != cudaSuccess) return prml_set_error(PRML_ERR_CUDA, std::string("prml_anti_laplacian launch: ") + cudaGetErrorString(e));
   long long its[PRML_JACOBI_MAX_BATCH];
