@@ -243,6 +243,55 @@ int prml_implicit_stop(const prml_implicit_params* p, const double* xs, const do
 int prml_implicit_finish(const prml_implicit_params* p, const double* x, const double* f, double* out,
                          void* stream);
 
+/* `count` secant iterations first, first + 1, .. of an implicit step, one
+ * launch each of a generated secant kernel (module with exact division,
+ * float64).  Iteration 0 only computes the residual of xa (the predictor
+ * p) into sec->q; iteration k >= 1 reads the current iterate (xb when k is
+ * odd, xa when it is even) and writes the next one to the other buffer.
+ * `base` holds the tables of the step's end; sec->x0 and sec->iteration are
+ * set per launch.  Before iteration 0: flags, predictor and second point as
+ * prml_implicit_predict leaves them, counters, done and stats zeroed. */
+int prml_secant_params_size(void);
+int prml_secant_run(void* kernel, int block, int tile_x, int tile_y, int box_rows, int box_cols, int comps,
+                    const prml_step_params* base, const prml_secant_params* sec, double* xa, double* xb,
+                    long long bstride, double t, int first, int count, void* stream);
+/* One whole implicit step (numerical_integrator.py:199-270) on `stream`:
+ * right-hand sides f0 at the step start, predictor, secant iterations until
+ * every instance has stopped or max_iterations, results to `out`.  The
+ * first `guess` iterations are issued at once, then half as many again (at
+ * least 8) between two reads of the counters.  words: device block of
+ * 7 batch (+ 1 if batch is odd) ints {counters, done} followed by 3 batch
+ * doubles (status sums), host_words its page-locked host copy, which holds
+ * the instances' iteration counts and sums on return.  `start` and `end` are the
+ * launch parameters with the boundary tables of the step's start and end. */
+typedef struct prml_secant_step {
+  void* rhs_kernel;
+  void* secant_kernel;
+  int rhs_tile[3], rhs_box[2];       /* rows, columns, threads; staged rows, columns */
+  int secant_tile[3], secant_box[2];
+  const prml_step_params* start;
+  const prml_step_params* end;
+  const prml_implicit_params* ip;
+  prml_secant_params sec;            /* y, fu, q, flags, res, a, dt, tol, kind    */
+  double* xa;
+  double* xb;
+  double* f0;
+  double* out;
+  int* words;
+  int* host_words;
+  const int* zero_counters;          /* [batch][4] zeros (prml_implicit_predict)  */
+  double t;
+  int guess, max_iterations;
+} prml_secant_step;
+int prml_secant_step_size(void);
+int prml_secant_solve(const prml_secant_step* step, void* stream);
+/* Finishes the instances still running after iteration k: xn the iterate
+ * that k wrote, xp the one before; with `force` (the iteration limit) those
+ * that k did not stop get xp, as the reference returns. */
+int prml_secant_stop(const prml_implicit_params* p, int k, const double* xn, const double* xp,
+                     const unsigned char* flags, const int* counters, int* done, int force, double* res,
+                     double* stats, void* stream);
+
 /* ---- layout conversion at the boundary ---------------------------------
  * The reference's state is a C-contiguous float64 array (*vertices, C)
  * (fdm_operator.py:53, solution.py:30-83); the kernels use planar padded

@@ -143,6 +143,36 @@ typedef struct prml_multi_params {
   int n_rounds;          /* largest n_steps of the groups                    */
 } prml_multi_params;
 
+/* ---- secant iterations of an implicit step --------------------------------
+ * One launch of a generated secant kernel (MODE 2 of the step body, float64)
+ * is one iteration of the reference's element-wise secant solve: the
+ * right-hand sides at the current iterate (the launch's stencil input), its
+ * residual, and the next iterate.  Iteration k also finishes the instances
+ * that iteration k - 1 stopped: their result, status sums and iteration
+ * count.  `counters` holds three sets of {some residual changed, some element
+ * stepped by tol or more} per instance, used in turn: iteration k writes set
+ * k % 3, reads set (k - 1) % 3 and clears set (k + 1) % 3. */
+#define PRML_SECANT_FAIL 1u   /* element flags: last step was tol or more (or none yet) */
+#define PRML_SECANT_ACTIVE 2u /* not yet set to a midpoint */
+#define PRML_SECANT_NZ 4u     /* residuals differed in the latest iteration */
+#define PRML_SECANT_MID 8u    /* set to a midpoint in the latest iteration */
+
+typedef struct prml_secant_params {
+  const double* y;       /* state at the step start                            */
+  const double* fu;      /* dt f at the step start (Crank-Nicolson)            */
+  double* x0;            /* previous iterate in, next iterate out              */
+  double* q;             /* previous residual in, this residual out            */
+  unsigned char* flags;  /* per element                                        */
+  int* counters;         /* [3][batch][2]                                      */
+  int* done;             /* [batch]: iteration that stopped the instance, or 0 */
+  double* res;           /* results of stopped instances                       */
+  double* stats;         /* [batch][3]: failing elements, failing with equal
+                            residuals, sum of squared moves of those           */
+  double a, dt, tol;
+  int crank_nicolson;
+  int iteration;         /* k >= 1, or 0: only the residual of the iterate     */
+} prml_secant_params;
+
 #ifdef __cplusplus
 }
 #endif

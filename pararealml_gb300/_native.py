@@ -145,6 +145,12 @@ def _declare(lib: ctypes.CDLL) -> None:
         "prml_implicit_status": (_c_int, [_p, _p, _p, _p, _p, _p]),
         "prml_implicit_stop": (_c_int, [_p, _p, _p, _p, _p, _p, _c_int, _p, _p, _p, _p]),
         "prml_implicit_finish": (_c_int, [_p, _p, _p, _p, _p]),
+        "prml_secant_params_size": (_c_int, []),
+        "prml_secant_run": (_c_int, [_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _p, _p, _p, _p, _c_ll, _c_d,
+                                     _c_int, _c_int, _p]),
+        "prml_secant_step_size": (_c_int, []),
+        "prml_secant_solve": (_c_int, [_p, _p]),
+        "prml_secant_stop": (_c_int, [_p, _c_int, _p, _p, _p, _p, _p, _c_int, _p, _p, _p]),
         "prml_measure_fp64_fma": (_c_int, [ctypes.POINTER(_c_d), _p]),
         "prml_gaussian_states": (_c_int, [_p, _c_ll, _c_int, _p, _c_int, _c_int, _p, _p]),
         "prml_multi_group_size": (_c_int, []),
@@ -207,6 +213,11 @@ def exported_symbols() -> list:
         "prml_implicit_status",
         "prml_implicit_stop",
         "prml_implicit_finish",
+        "prml_secant_params_size",
+        "prml_secant_run",
+        "prml_secant_step_size",
+        "prml_secant_solve",
+        "prml_secant_stop",
         "prml_measure_fp64_fma",
         "prml_gaussian_states",
         "prml_multi_group_size",
@@ -385,6 +396,27 @@ class JacobiParams(ctypes.Structure):
     ]
 
 
+class SecantParams(ctypes.Structure):
+    """Mirror of ``prml_secant_params`` (include/prml_params.h)."""
+
+    _fields_ = [
+        ("y", _p),
+        ("fu", _p),
+        ("x0", _p),
+        ("q", _p),
+        ("flags", _p),
+        ("counters", _p),
+        ("done", _p),
+        ("res", _p),
+        ("stats", _p),
+        ("a", _c_d),
+        ("dt", _c_d),
+        ("tol", _c_d),
+        ("crank_nicolson", _c_int),
+        ("iteration", _c_int),
+    ]
+
+
 class ImplicitParams(ctypes.Structure):
     """Mirror of ``prml_implicit_params`` (include/pararealml_gb300.h)."""
 
@@ -406,6 +438,33 @@ class ImplicitParams(ctypes.Structure):
         ("a", _c_d),
         ("tol", _c_d),
         ("dx", _c_d),
+    ]
+
+
+class SecantStep(ctypes.Structure):
+    """Mirror of ``prml_secant_step`` (include/pararealml_gb300.h)."""
+
+    _fields_ = [
+        ("rhs_kernel", _p),
+        ("secant_kernel", _p),
+        ("rhs_tile", _c_int * 3),
+        ("rhs_box", _c_int * 2),
+        ("secant_tile", _c_int * 3),
+        ("secant_box", _c_int * 2),
+        ("start", ctypes.POINTER(StepParams)),
+        ("end", ctypes.POINTER(StepParams)),
+        ("ip", ctypes.POINTER(ImplicitParams)),
+        ("sec", SecantParams),
+        ("xa", _p),
+        ("xb", _p),
+        ("f0", _p),
+        ("out", _p),
+        ("words", _p),
+        ("host_words", _p),
+        ("zero_counters", _p),
+        ("t", _c_d),
+        ("guess", _c_int),
+        ("max_iterations", _c_int),
     ]
 
 

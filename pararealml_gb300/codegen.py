@@ -20,6 +20,7 @@ doubles that the reference's lambdified numpy code uses.
 from __future__ import annotations
 
 import dataclasses
+import functools
 import hashlib
 from typing import Dict, List, Sequence, Tuple
 
@@ -85,6 +86,9 @@ TILE_CONFIGS_3D: Tuple[Tuple[int, int, int, int, int], ...] = (
     (4, 16, 128, 1, 2),
     (2, 16, 64, 1, 2),
 )
+# tile of the secant-iteration kernel on 0-2D meshes: 257^2 diffusion 15.9 us per
+# iteration; 16.9 us with 2 x 64, 18-27 us with other shapes of 64 to 512 vertices
+SECANT_TILE: Tuple[int, int, int] = (8, 32, 256)
 SMEM_LIMIT = 227 * 1024
 # tiles of the multi-round kernels (one cooperative launch takes every step
 # of several groups of instances, a grid barrier between rounds)
@@ -828,10 +832,12 @@ class GeneratedModule:
     rhs_kernel: Tuple[str, int, Tuple[int, int, int]]
     n_comp: int = 1
     multi_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
+    # secant-iteration kernel of modules with exact division: (name, smem, tile)
+    secant_kernel: Tuple[str, int, tuple] = None
     # marching kernels: tile (jobs per SM, cols, threads, steps, 0, "m", columns per lane) -> (name, smem)
     march_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
 
-    @property
+    @functools.cached_property
     def kernels(self) -> Dict[tuple, Tuple[str, int]]:
         """Every step kernel: tile -> (name, dynamic shared memory)."""
         return {**self.step_kernels, **self.march_kernels}
@@ -885,6 +891,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
     # whether any right-hand side reads t (else the kernels skip time arithmetic)
     uses_t = any(sym.name == "t" for expr in low.rhs for sym in expr.free_symbols)
     d_rows, y_rows = list(low.d_idx), list(low.y_idx)
+    side_mask, corners = _side_columns(low)
     three_d = low.x_dimension == 3
     if three_d and comp:
         raise NotImplementedError("compensated float32 is not available on 3D meshes")
@@ -900,12 +907,12 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         f"  static constexpr bool EXACT_DIV = {'true' if exact_div else 'false'};",
         f"  static constexpr bool FAST = {'true' if fast else 'false'};",
         f"  static constexpr bool EQUAL_DX = {'true' if low.dx_k[0] == low.dx_k[1] else 'false'};",
-        f"  static constexpr unsigned HMASK = {_side_columns(low)[0]}u;",
-        f"  static constexpr bool CORNERS = {'true' if _side_columns(low)[1] else 'false'};",
+        f"  static constexpr unsigned HMASK = {side_mask}u;",
+        f"  static constexpr bool CORNERS = {'true' if corners else 'false'};",
         f"  static constexpr bool DYNAMIC = {'true' if low.dynamic else 'false'};",
         # column-face values may be read once per row: static conditions, no
         # mixed derivative, and no lane that touches both column faces
-        f"  static constexpr bool PRE = {'true' if not low.dynamic and not _side_columns(low)[1] and low.ny > 8 else 'false'};",
+        f"  static constexpr bool PRE = {'true' if not low.dynamic and not corners and low.ny > 8 else 'false'};",
         f"  static constexpr unsigned long long NEU_MASK = {low.neu_mask}ull;",
         f"  static constexpr unsigned long long DIR_MASK = {low.dir_mask}ull;",
         f"  static __device__ constexpr int dcomp(int i) {{ return {_chain(d_rows)}; }}",
@@ -941,10 +948,21 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
             f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin) "
             f"{{ prml::step_body3<{ctype}, Eq, {integrator}, {rtile[4]}, {rtile[0]}, {rtile[1]}, {rtile[2]}, 1>(p, tin); }}"
         )
+        secant = None
+        if exact_div and ctype == "double":
+            sname = kernel_name("secant", dtype, rtile)
+            secant = (sname, rsm, rtile)
+            body.append(
+                f'extern "C" __global__ void __launch_bounds__({rtile[2]}) {sname}'
+                f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin, const prml_secant_params s) "
+                f"{{ prml::step_body3<{ctype}, Eq, {integrator}, {rtile[4]}, {rtile[0]}, {rtile[1]}, {rtile[2]}, 2>"
+                f"(p, tin, &s); }}"
+            )
         source = "\n".join(body) + "\n"
         key = hashlib.sha256((source + _template_digest()).encode()).hexdigest()[:24]
         return GeneratedModule(source=source, key=key, dtype=dtype, integrator=integrator, invariant=invariant,
-                               step_kernels=step_kernels, rhs_kernel=(rname, rsm, rtile), n_comp=low.n_comp)
+                               step_kernels=step_kernels, rhs_kernel=(rname, rsm, rtile), n_comp=low.n_comp,
+                               secant_kernel=secant)
     # temporally blocked kernels take several steps per launch; a Jacobi
     # solve has to run between every two steps
     blocked = single_stage and not low.lap_idx
@@ -1004,6 +1022,17 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin) "
         f"{{ prml::step_body<{ctype}, Eq, {integrator}, {rtile[0]}, {rtile[1]}, {rtile[2]}, 1>(p, tin); }}"
     )
+    # secant iterations of an implicit step
+    secant = None
+    if exact_div and ctype == "double":
+        stile = SECANT_TILE
+        sname = kernel_name("secant", dtype, stile)
+        secant = (sname, smem_bytes(low, integrator, invariant, stile, esize, 1), stile)
+        body.append(
+            f'extern "C" __global__ void __launch_bounds__({stile[2]}) {sname}'
+            f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin, const prml_secant_params s) "
+            f"{{ prml::step_body<{ctype}, Eq, {integrator}, {stile[0]}, {stile[1]}, {stile[2]}, 2>(p, tin, &s); }}"
+        )
     # multi-round kernels: every step of several groups in one cooperative
     # launch (not for Jacobi rows, which need a solve between two steps)
     multi_kernels = {}
@@ -1031,4 +1060,5 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         n_comp=low.n_comp,
         multi_kernels=multi_kernels,
         march_kernels=march_kernels,
+        secant_kernel=secant,
     )

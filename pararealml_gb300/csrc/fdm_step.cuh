@@ -98,6 +98,22 @@ __device__ __forceinline__ T fmaT(T a, T b, T c) {
   else return __fma_rn(a, b, c);
 }
 
+/* x / d for a divisor whose reciprocal y = RN(1 / d) is known: the product
+ * x y, and two corrections by the remainder.  The first makes the quotient
+ * faithful, the second correctly rounded (Markstein, "Computation of
+ * elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+ * Dev. 34, 1990: the theorem on the final correction).  Five float64 operations
+ * instead of a general division's; arguments near the ends of the exponent
+ * range (and zeros) divide. */
+__device__ __forceinline__ double quot(double x, double d, double y) {
+  const unsigned e = (unsigned)__double2hiint(x) & 0x7ff00000u;
+  if (e - 0x10000000u >= 0x60000000u) return __ddiv_rn(x, d);
+  double q = __dmul_rn(x, y);
+  q = __fma_rn(__fma_rn(-q, d, x), y, q);
+  return __fma_rn(__fma_rn(-q, d, x), y, q);
+}
+__device__ __forceinline__ float quot(float x, float d, float) { return x / d; }
+
 /* A vertex of the current stage input, with the stencil operators the
  * generated right-hand sides call. */
 template <typename T, class Eq, int RY, int RXY, bool EDGE = true>
@@ -141,7 +157,7 @@ struct Point {
         const T g = face(m->neu, 1, c, qj);
         if (g == g) return g;
       }
-      if constexpr (Eq::EXACT_DIV) return (v(c, di + 1, dj) - v(c, di - 1, dj)) / m->twod0;
+      if constexpr (Eq::EXACT_DIV) return quot(v(c, di + 1, dj) - v(c, di - 1, dj), m->twod0, m->inv2d0);
       return (v(c, di + 1, dj) - v(c, di - 1, dj)) * m->inv2d0;
     } else {
       if (EDGE && has_neu(2, c) && qj == 0) {
@@ -152,7 +168,7 @@ struct Point {
         const T g = face(m->neu, 3, c, qi);
         if (g == g) return g;
       }
-      if constexpr (Eq::EXACT_DIV) return (v(c, di, dj + 1) - v(c, di, dj - 1)) / m->twod1;
+      if constexpr (Eq::EXACT_DIV) return quot(v(c, di, dj + 1) - v(c, di, dj - 1), m->twod1, m->inv2d1);
       return (v(c, di, dj + 1) - v(c, di, dj - 1)) * m->inv2d1;
     }
   }
@@ -195,10 +211,10 @@ struct Point {
     T prev, next;
     ends<c, ka>(prev, next);
     if (ka == 0) {
-      if constexpr (Eq::EXACT_DIV) return ((next - T(2) * mid) + prev) / m->dd0;
+      if constexpr (Eq::EXACT_DIV) return quot(fmaT(T(-2), mid, next) + prev, m->dd0, m->invdd0);
       return ((next - T(2) * mid) + prev) * m->invdd0;
     } else {
-      if constexpr (Eq::EXACT_DIV) return ((next - T(2) * mid) + prev) / m->dd1;
+      if constexpr (Eq::EXACT_DIV) return quot(fmaT(T(-2), mid, next) + prev, m->dd1, m->invdd1);
       return ((next - T(2) * mid) + prev) * m->invdd1;
     }
   }
@@ -233,8 +249,8 @@ struct Point {
   template <int c, int a1, int a2> __device__ __forceinline__ T hess() const {
     if (a1 == a2) return sd<c, a1>();
     if constexpr (Eq::EXACT_DIV) {
-      if (a2 == 0) return (grad_at<c, a1, true>(1, 0) - grad_at<c, a1, true>(-1, 0)) / m->twod0;
-      return (grad_at<c, a1, true>(0, 1) - grad_at<c, a1, true>(0, -1)) / m->twod1;
+      if (a2 == 0) return quot(grad_at<c, a1, true>(1, 0) - grad_at<c, a1, true>(-1, 0), m->twod0, m->inv2d0);
+      return quot(grad_at<c, a1, true>(0, 1) - grad_at<c, a1, true>(0, -1), m->twod1, m->inv2d1);
     }
     if (a2 == 0)
       return (grad_at<c, a1, true>(1, 0) - grad_at<c, a1, true>(-1, 0)) * m->inv2d0;
@@ -443,6 +459,119 @@ __device__ __forceinline__ T step_result(T y, T acc, T acc_scale) {
   else return (INTEG == RK4) ? y + div6(acc) : y + acc;
 }
 
+/* ---- secant iterations (prml_secant_params) ------------------------------ */
+
+/* Result and status of one element of an instance that iteration k stopped:
+ * xs its new iterate, xo the iterate before (numerical_integrator.py:
+ * 199-270).  Where no residual changed at all every element goes to the
+ * midpoint; those not set to one in that iteration are moved here. */
+struct SecantTally {
+  int fail, zero;
+  double rms2;
+};
+__device__ __forceinline__ double secant_result(double xs, double xo, unsigned fl, bool flat, SecantTally& t) {
+  const double v = (flat && !(fl & PRML_SECANT_MID)) ? __ddiv_rn(__dadd_rn(xo, xs), 2.0) : xs;
+  if (fl & PRML_SECANT_FAIL) {
+    ++t.fail;
+    if (!(fl & PRML_SECANT_NZ)) {
+      ++t.zero;
+      const double d = xo - v;
+      if (xo != v) t.rms2 += d * d;
+    }
+  }
+  return v;
+}
+__device__ __forceinline__ void secant_report(double* stats, SecantTally t) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t.fail += __shfl_xor_sync(0xffffffffu, t.fail, o);
+    t.zero += __shfl_xor_sync(0xffffffffu, t.zero, o);
+  }
+  if ((threadIdx.x & 31) == 0 && t.fail) atomicAdd(stats, (double)t.fail);
+  if ((threadIdx.x & 31) == 0 && t.zero) atomicAdd(stats + 1, (double)t.zero);
+  if (t.rms2 != 0.0) atomicAdd(stats + 2, t.rms2);
+}
+
+/* Operands of one element besides the stencil input, read before the wait for
+ * the tile so that their latency overlaps the copy's. */
+struct SecantIn {
+  double y, fu, x0, q;
+  unsigned fl;
+};
+__device__ __forceinline__ SecantIn secant_load(const prml_secant_params& s, long long e) {
+  SecantIn r;
+  r.y = __ldcg(s.y + e);
+  r.fu = s.crank_nicolson ? __ldcg(s.fu + e) : 0.0;
+  r.x0 = s.iteration ? __ldcg(s.x0 + e) : 0.0;
+  r.q = s.iteration ? __ldcg(s.q + e) : 0.0;
+  r.fl = s.iteration ? __ldcg(s.flags + e) : 0u;
+  return r;
+}
+
+/* One element: the residual r of the current iterate x1 and the secant step.
+ * The step assumes that some residual of the instance changed; if none did,
+ * every element took the midpoint branch and secant_result completes it. */
+__device__ __forceinline__ void secant_element(const prml_secant_params& s, long long e, const SecantIn& in, double x1,
+                                               double r, bool& changed, bool& failing) {
+  s.q[e] = r;
+  if (s.iteration == 0) return;
+  unsigned fl = in.fl;
+  if (r != in.q) {
+    changed = true;
+    const double step = __ddiv_rn(__dmul_rn(r, __dsub_rn(x1, in.x0)), __dsub_rn(r, in.q));
+    s.x0[e] = __dsub_rn(x1, step);
+    const bool fail = fabs(step) >= s.tol;
+    failing |= fail;
+    fl = (fl & PRML_SECANT_ACTIVE) | PRML_SECANT_NZ | (fail ? PRML_SECANT_FAIL : 0u);
+  } else {
+    const bool mid = fl & PRML_SECANT_ACTIVE;
+    if (mid) s.x0[e] = __ddiv_rn(__dadd_rn(x1, in.x0), 2.0);
+    fl = (fl & PRML_SECANT_FAIL) | (mid ? PRML_SECANT_MID : 0u); /* inactive from now on, failure state kept */
+  }
+  s.flags[e] = (unsigned char)fl;
+}
+
+/* y + (a dt) f + (1 - a) fu, or y + dt f: what the residual subtracts from the
+ * iterate after the constraints, rounded like the numpy expressions. */
+__device__ __forceinline__ double secant_target(const prml_secant_params& s, const SecantIn& in, double f) {
+  if (s.crank_nicolson)
+    return __dadd_rn(__dadd_rn(in.y, __dmul_rn(__dmul_rn(s.a, s.dt), f)), __dmul_rn(1.0 - s.a, in.fu));
+  return __dadd_rn(in.y, __dmul_rn(s.dt, f));
+}
+
+/* Per tile of instance b (tile 0 of the instance: `first`): what to do, and
+ * whether iteration k - 1 changed no residual.  The mark set here only becomes
+ * "earlier" for iteration k + 1. */
+enum { SECANT_ITERATE = 0, SECANT_FINISH = 1, SECANT_IDLE = 2 };
+__device__ __forceinline__ int secant_tile(const prml_secant_params& s, int batch, int b, bool first, bool& flat) {
+  flat = false;
+  if (s.iteration < 2) return SECANT_ITERATE;
+  const int prev = s.iteration - 1;
+  const int* c = s.counters + ((prev % 3) * batch + b) * 2;
+  const int d = *(volatile const int*)(s.done + b), changed = __ldcg(c), failing = __ldcg(c + 1);
+  if (d && d < prev) return SECANT_IDLE;
+  if (changed && failing) return SECANT_ITERATE;
+  flat = !changed;
+  if (first && threadIdx.x == 0) *(volatile int*)(s.done + b) = prev;
+  return SECANT_FINISH;
+}
+/* The counters of iteration k after a tile (every lane of the warp calls). */
+__device__ __forceinline__ void secant_count(const prml_secant_params& s, int batch, int b, bool changed, bool failing) {
+  if (s.iteration == 0) return;
+  int* cnt = s.counters + ((s.iteration % 3) * batch + b) * 2;
+  const bool ch = __any_sync(0xffffffffu, changed), fa = __any_sync(0xffffffffu, failing);
+  if ((threadIdx.x & 31) == 0) {
+    if (ch) cnt[0] = 1;
+    if (fa) cnt[1] = 1;
+  }
+}
+
+/* Clears the counter set of the next iteration (block 0). */
+__device__ __forceinline__ void secant_clear(const prml_secant_params& s, int batch) {
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < 2 * batch; k += blockDim.x) s.counters[((s.iteration + 1) % 3) * 2 * batch + k] = 0;
+}
+
 /* Stage-and-combine work of one tile whose input (tile + halo) is already
  * in `ybuf`.  MODE 0: one integrator step.  MODE 1: write the right-hand
  * side of every equation (dy/dt for D_Y_OVER_D_T rows, the value for LHS.Y
@@ -621,6 +750,65 @@ __device__ __forceinline__ void tile_compute(const prml_step_params& p, const Me
   }
 }
 
+/* The operands of a tile's elements (this thread's), see secant_load. */
+template <int C, int PER, int TX, int TY, int NT>
+__device__ __forceinline__ void secant_prefetch(const prml_step_params& p, const prml_secant_params& s, int b, int gi0,
+                                                int gj0, SecantIn (&in)[PER][C]) {
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int k = threadIdx.x + q * NT;
+    const int gi = gi0 + k / TY, gj = gj0 + k % TY;
+    if (gi >= p.nx || gj >= p.ny) continue;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      in[q][c] = secant_load(s, (long long)b * p.in_bstride + c * p.cstride + (long long)gi * p.pitch + gj);
+  }
+}
+
+/* One secant iteration on one staged tile of the current iterate. */
+template <typename T, class Eq, int PER, int TX, int TY, int NT, bool EDGE>
+__device__ __forceinline__ void tile_secant(const prml_step_params& p, const MeshC<T>& m, const T* ybuf, int b, int gi0,
+                                            int gj0, const prml_secant_params& s, int what, bool flat,
+                                            const SecantIn (&in)[PER][Eq::C]) {
+  constexpr int C = Eq::C;
+  constexpr int ND = Eq::ND;
+  constexpr int HX = 1, HY = ColHalo<T, 1>::value;
+  constexpr int RY = TY + 2 * HY, RXY = (TX + 2 * HX) * RY;
+  const double t = Eq::USES_T ? p.t + (p.t_offset ? p.t_offset[b] : 0.0) : 0.0;
+  bool changed = false, failing = false;
+  SecantTally tally{0, 0, 0.0};
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int k = threadIdx.x + q * NT;
+    const int ti = k / TY, tj = k % TY;
+    const int gi = gi0 + ti, gj = gj0 + tj;
+    if (EDGE && (gi >= p.nx || gj >= p.ny)) continue;
+    const int l = (HX + ti) * RY + HY + tj;
+    T f[ND > 0 ? ND : 1];
+    if (what == SECANT_ITERATE && ND > 0) {
+      Point<T, Eq, RY, RXY, EDGE> pt{ybuf, l, gi, gj, &m, t};
+      Eq::rhs_dt(pt, f);
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const long long e = (long long)b * p.in_bstride + c * p.cstride + (long long)gi * p.pitch + gj;
+      const T x1 = ybuf[c * RXY + l];
+      if (what == SECANT_FINISH) {
+        s.res[e] = secant_result(x1, in[q][c].x0, in[q][c].fl, flat, tally);
+        continue;
+      }
+      T fc = T(0);
+#pragma unroll
+      for (int i = 0; i < ND; ++i)
+        if (Eq::dcomp(i) == c) fc = f[i];
+      const T target = dirichlet<T, Eq, EDGE>(secant_target(s, in[q][c], fc), c, gi, gj, m);
+      secant_element(s, e, in[q][c], x1, __dsub_rn(x1, target), changed, failing);
+    }
+  }
+  if (what == SECANT_FINISH) secant_report(s.stats + 3 * b, tally);
+  else secant_count(s, p.batch, b, changed, failing);
+}
+
 /* Single-stage time steps on one staged tile, in one pass per step: the
  * right-hand sides, the LHS.Y values, the combination, the Dirichlet values
  * and the store of each vertex together.  TB > 1 (temporal blocking):
@@ -770,11 +958,18 @@ __device__ __forceinline__ void tile_compute_tb(const prml_step_params& p, const
  * on the GPU at once, and each CTA walks the tiles (all instances, row-major
  * within an instance) with a stride of gridDim.x.  The input of the next
  * tile is fetched by TMA into the second staging buffer while the current
- * tile is computed, so load latency overlaps compute. */
+ * tile is computed, so load latency overlaps compute.  MODE 2: one secant
+ * iteration of an implicit step (prml_secant_params; float64), one launch
+ * where right-hand side, residual, update, stop test and result copy were
+ * five: 15.9 us per iteration at 257^2 (diffusion, backward Euler), 45 us
+ * before.  The launch chain with its loads takes 6 us of it (an idle iteration),
+ * the rest the float64 pipe: about 35 operations per vertex, ten of them the
+ * secant's division. */
 template <typename T, class Eq, int INTEG, int TX, int TY, int NT, int MODE, int COMP = 0, int TB = 1>
-__device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDesc& tin) {
+__device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDesc& tin,
+                                          const prml_secant_params* sec = nullptr) {
   constexpr int C = Eq::C;
-  constexpr int NSTAGE = (MODE == 1 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
+  constexpr int NSTAGE = (MODE != 0 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
   static_assert(TB == 1 || (MODE == 0 && NSTAGE == 1), "temporal blocking needs single-stage steps");
   static_assert(TB >= 1 && TB <= PRML_TB_MAX, "temporal block out of range");
   constexpr int HX = TB > 1 ? TB : NSTAGE;
@@ -873,6 +1068,7 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
    * launch did not ask for the overlap. */
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if constexpr (MODE == 2) secant_clear(*sec, p.batch);
   __syncthreads();
   int t = blockIdx.x;
   Walk cur;
@@ -888,6 +1084,14 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
     /* the other staging buffer was released by the __syncthreads that ended
      * the previous iteration */
     if (threadIdx.x == 0 && next < total) issue(nxt, buf ^ 1);
+    constexpr int PER = (TX * TY) / NT;
+    SecantIn sec_in[MODE == 2 ? PER : 1][C];
+    int sec_what = 0;
+    bool sec_flat = false;
+    if constexpr (MODE == 2) {
+      sec_what = secant_tile(*sec, p.batch, cur.b, cur.ty == 0 && cur.tx == 0, sec_flat);
+      secant_prefetch<C, PER, TX, TY, NT>(p, *sec, cur.b, cur.ty * TX, cur.tx * TY, sec_in);
+    }
     const bool ok = mbar_wait_bounded(&bar[buf], (unsigned)((it >> 1) & 1), wait_ns);
     if (__syncthreads_or(!ok)) {
       /* a copy did not land in time: report, let in-flight copies finish
@@ -904,7 +1108,12 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
      * face (Neumann, Dirichlet) and inside tests compile away */
     const bool edge = gi0 < HX + 1 || gi0 + TX + HX + 1 > p.nx || gj0 < HX + 1 || gj0 + TY + HX + 1 > p.ny;
     const T* ybuf = buf ? ybuf1 : ybuf0;
-    if constexpr (MODE == 0 && NSTAGE == 1) {
+    if constexpr (MODE == 2) {
+      if (sec_what != SECANT_IDLE) {
+        if (edge) tile_secant<T, Eq, PER, TX, TY, NT, true>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in);
+        else tile_secant<T, Eq, PER, TX, TY, NT, false>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in);
+      }
+    } else if constexpr (MODE == 0 && NSTAGE == 1) {
       /* single-stage steps (one or TB per launch): one pass per step */
       if (edge) tile_compute_tb<T, Eq, INTEG, TX, TY, NT, TB, COMP, true>(p, m, ybuf, bufA, bufB, b, gi0, gj0);
       else tile_compute_tb<T, Eq, INTEG, TX, TY, NT, TB, COMP, false>(p, m, ybuf, bufA, bufB, b, gi0, gj0);

@@ -83,7 +83,8 @@ struct Point3 {
       if (gv == gv) return gv;
     }
     const int e0 = ka == 0, e1 = ka == 1, e2 = ka == 2;
-    if constexpr (Eq::EXACT_DIV) return (v(c, d0 + e0, d1 + e1, d2 + e2) - v(c, d0 - e0, d1 - e1, d2 - e2)) / m->twod[ka];
+    if constexpr (Eq::EXACT_DIV)
+      return quot(v(c, d0 + e0, d1 + e1, d2 + e2) - v(c, d0 - e0, d1 - e1, d2 - e2), m->twod[ka], m->inv2d[ka]);
     return (v(c, d0 + e0, d1 + e1, d2 + e2) - v(c, d0 - e0, d1 - e1, d2 - e2)) * m->inv2d[ka];
   }
   template <int c, int ka> __device__ __forceinline__ T grad() const { return grad_at<c, ka, false>(0, 0, 0); }
@@ -101,7 +102,7 @@ struct Point3 {
       const T gv = face(m->neu, 2 * ka + 1, c, g[0], g[1], g[2]);
       if (gv == gv) next = lo + m->twod[ka] * gv;
     }
-    if constexpr (Eq::EXACT_DIV) return ((next - T(2) * mid) + prev) / m->dd[ka];
+    if constexpr (Eq::EXACT_DIV) return quot(fmaT(T(-2), mid, next) + prev, m->dd[ka], m->invdd[ka]);
     return ((next - T(2) * mid) + prev) * m->invdd[ka];
   }
 
@@ -109,7 +110,8 @@ struct Point3 {
   template <int c, int a1, int a2> __device__ __forceinline__ T hess() const {
     if (a1 == a2) return sd<c, a1>();
     const int e0 = a2 == 0, e1 = a2 == 1, e2 = a2 == 2;
-    if constexpr (Eq::EXACT_DIV) return (grad_at<c, a1, true>(e0, e1, e2) - grad_at<c, a1, true>(-e0, -e1, -e2)) / m->twod[a2];
+    if constexpr (Eq::EXACT_DIV)
+      return quot(grad_at<c, a1, true>(e0, e1, e2) - grad_at<c, a1, true>(-e0, -e1, -e2), m->twod[a2], m->inv2d[a2]);
     return (grad_at<c, a1, true>(e0, e1, e2) - grad_at<c, a1, true>(-e0, -e1, -e2)) * m->inv2d[a2];
   }
 };
@@ -152,10 +154,11 @@ __device__ __forceinline__ void tma_load_5d3(void* dst, const TmaDesc* map, int 
  * the right-hand sides).  Same schedule as the 2D tile_compute. */
 template <typename T, class Eq, int INTEG, int TZ, int TX, int TY, int NT, int MODE>
 __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const MeshC3<T>& m, const T* ybuf,
-                                              T* bufA, T* bufB, int b, int gk0, int gi0, int gj0) {
+                                              T* bufA, T* bufB, int b, int gk0, int gi0, int gj0,
+                                              const prml_secant_params* sec = nullptr) {
   constexpr int C = Eq::C;
   constexpr int ND = Eq::ND;
-  constexpr int NSTAGE = (MODE == 1 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
+  constexpr int NSTAGE = (MODE != 0 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
   constexpr int HZ = NSTAGE, HX = NSTAGE, HY = ColHalo<T, NSTAGE>::value;
   constexpr int RZ = TZ + 2 * HZ, RX = TX + 2 * HX, RY = TY + 2 * HY, RXY = RX * RY, RV = RZ * RXY;
   constexpr int PER = (TZ * TX * TY) / NT;
@@ -170,6 +173,13 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
   const T* cur = ybuf;
   T* nxt = bufA;
   (void)bufB;
+  int sec_what = 0;
+  bool sec_changed = false, sec_failing = false, sec_flat = false;
+  SecantTally sec_tally{0, 0, 0.0};
+  if constexpr (MODE == 2) {
+    sec_what = secant_tile(*sec, p.batch, b, gk0 == 0 && gi0 == 0 && gj0 == 0, sec_flat);
+    if (sec_what == SECANT_IDLE) return;
+  }
 
 #pragma unroll
   for (int s = 0; s < NSTAGE; ++s) {
@@ -192,6 +202,27 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
         return;
       }
       P pt{cur, l, {g[0], g[1], g[2]}, &ms, ts};
+      if constexpr (MODE == 2) {
+        T f[ND > 0 ? ND : 1];
+        if (sec_what == SECANT_ITERATE && ND > 0) Eq::rhs_dt(pt, f);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const long long e = (long long)b * p.in_bstride + c * p.cstride + g[0] * plane + (long long)g[1] * p.pitch + g[2];
+          const T x1 = cur[c * RV + l]; /* the current iterate */
+          const SecantIn in = secant_load(*sec, e);
+          if (sec_what == SECANT_FINISH) {
+            sec->res[e] = secant_result(x1, in.x0, in.fl, sec_flat, sec_tally);
+            continue;
+          }
+          T fc = T(0);
+#pragma unroll
+          for (int i = 0; i < ND; ++i)
+            if (Eq::dcomp(i) == c) fc = f[i];
+          const T target = dirichlet3<T, Eq>(secant_target(*sec, in, fc), c, g, ms);
+          secant_element(*sec, e, in, x1, __dsub_rn(x1, target), sec_changed, sec_failing);
+        }
+        return;
+      }
       if (MODE == 1) {
         T f[ND > 0 ? ND : 1];
         T gy[Eq::NYC > 0 ? Eq::NYC : 1];
@@ -274,7 +305,11 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
       nxt = (nxt == bufA) ? bufB : bufA;
     }
   }
-  if (MODE == 1) return;
+  if constexpr (MODE == 2) {
+    if (sec_what == SECANT_FINISH) secant_report(sec->stats + 3 * b, sec_tally);
+    else secant_count(*sec, p.batch, b, sec_changed, sec_failing);
+  }
+  if (MODE != 0) return;
 
   /* final combination, LHS.Y rows (at t with the step-start Neumann values),
    * Dirichlet at t + dt, store */
@@ -313,9 +348,10 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
  * a stride of gridDim.x; the next tile's box is loaded by TMA into the
  * other staging buffer while the current one is computed. */
 template <typename T, class Eq, int INTEG, int TZ, int TX, int TY, int NT, int MODE>
-__device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaDesc& tin) {
+__device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaDesc& tin,
+                                           const prml_secant_params* sec = nullptr) {
   constexpr int C = Eq::C;
-  constexpr int NSTAGE = (MODE == 1 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
+  constexpr int NSTAGE = (MODE != 0 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
   constexpr int HZ = NSTAGE, HX = NSTAGE, HY = ColHalo<T, NSTAGE>::value;
   constexpr int RZ = TZ + 2 * HZ, RX = TX + 2 * HX, RY = TY + 2 * HY;
   constexpr int NSTG = NSTAGE == 1 ? 0 : (NSTAGE == 2 ? 1 : 2);
@@ -396,6 +432,7 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if constexpr (MODE == 2) secant_clear(*sec, p.batch);
   __syncthreads();
   int t = blockIdx.x;
   if (threadIdx.x == 0 && t < total) issue(t, 0);
@@ -414,7 +451,7 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
     int b, tz, ty, tx;
     coords(t, b, tz, ty, tx);
     tile_compute3<T, Eq, INTEG, TZ, TX, TY, NT, MODE>(p, m, buf ? ybuf1 : ybuf0, bufA, bufB, b, tz * TZ,
-                                                     ty * TX, tx * TY);
+                                                     ty * TX, tx * TY, sec);
     __syncthreads();
   }
 }

@@ -417,8 +417,8 @@ int prml_set_step_overlap(int enabled) {
 }
 
 static int launch_step(Kernel* k, int block, int grid, prml_step_params* p, CUtensorMap* map,
-                       CUstream stream) {
-  void* args[] = {p, map};
+                       CUstream stream, prml_secant_params* sec = nullptr) {
+  void* args[] = {p, map, sec};
   CUresult r;
   if (g_step_overlap && g_drv.LaunchKernelEx) {
     CUlaunchAttribute attr[1];
@@ -689,6 +689,98 @@ int prml_fdm_rhs(void* kernel, int block, int tile_x, int tile_y, int box_rows, 
   rc = persistent_grid(k, block, base, tile_x, tile_y, &grid);
   if (rc) return rc;
   return launch_step(k, block, grid, &p, &map, static_cast<CUstream>(stream));
+}
+
+int prml_secant_params_size(void) { return (int)sizeof(prml_secant_params); }
+
+int prml_secant_run(void* kernel, int block, int tile_x, int tile_y, int box_rows, int box_cols, int comps,
+                    const prml_step_params* base, const prml_secant_params* sec, double* xa, double* xb,
+                    long long bstride, double t, int first, int count, void* stream) {
+  Kernel* k = static_cast<Kernel*>(kernel);
+  if (!k || !sec || !xa || !xb) return fail(PRML_ERR_ARG, "prml_secant_run: null argument");
+  int rc = check_geometry(base, tile_x, tile_y, block);
+  if (rc) return rc;
+  if (first < 0 || count < 0 || comps < 1 || base->elem_bytes != 8)
+    return fail(PRML_ERR_ARG, "prml_secant_run: bad iteration range or element type");
+  if (!sec->y || !sec->q || !sec->flags || !sec->counters || !sec->done || !sec->res || !sec->stats ||
+      (sec->crank_nicolson && !sec->fu))
+    return fail(PRML_ERR_ARG, "prml_secant_run: null buffer");
+  CUtensorMap maps[2];
+  for (int i = 0; i < 2; ++i) {
+    rc = encode_state_map(&maps[i], base, i ? xb : xa, bstride, bstride * base->batch, 1, box_rows, box_cols, comps);
+    if (rc) return rc;
+  }
+  int grid = 0;
+  rc = persistent_grid(k, block, base, tile_x, tile_y, &grid);
+  if (rc) return rc;
+  prml_step_params p = *base;
+  prml_secant_params s = *sec;
+  p.in_slot = 0;
+  p.in_bstride = bstride;
+  p.t = t;
+  for (int it = first; it < first + count; ++it) {
+    /* the iterates swap roles: iteration 1 reads xb and writes xa */
+    p.in = (it & 1) ? xb : xa;
+    s.x0 = (it & 1) ? xa : xb;
+    s.iteration = it;
+    rc = launch_step(k, block, grid, &p, &maps[it & 1], static_cast<CUstream>(stream), &s);
+    if (rc) return rc;
+  }
+  return PRML_OK;
+}
+
+int prml_secant_step_size(void) { return (int)sizeof(prml_secant_step); }
+
+int prml_secant_solve(const prml_secant_step* a, void* stream) {
+  if (!a || !a->start || !a->end || !a->ip || !a->xa || !a->xb || !a->f0 || !a->out || !a->words || !a->host_words ||
+      !a->zero_counters || a->max_iterations < 1)
+    return fail(PRML_ERR_ARG, "prml_secant_solve: bad argument");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int nb = a->start->batch, C = a->ip->comps;
+  const long long inst = a->ip->inst;
+  const size_t ints = 7 * (size_t)nb + (nb & 1), bytes = 4 * ints + 24 * (size_t)nb;
+  prml_secant_params sec = a->sec;
+  sec.counters = a->words;
+  sec.done = a->words + 6 * nb;
+  sec.stats = reinterpret_cast<double*>(a->words + ints);
+  cudaError_t e = cudaMemsetAsync(a->words, 0, bytes, st);
+  if (e != cudaSuccess) return fail(PRML_ERR_CUDA, std::string("prml_secant_solve: ") + cudaGetErrorString(e));
+  int rc = prml_fdm_rhs(a->rhs_kernel, a->rhs_tile[2], a->rhs_tile[0], a->rhs_tile[1], a->rhs_box[0], a->rhs_box[1], C,
+                        a->start, sec.y, inst, a->f0, inst, a->t, stream);
+  if (rc) return rc;
+  rc = prml_implicit_predict(a->ip, sec.y, a->f0, const_cast<double*>(sec.fu), a->xa, a->xb, sec.flags,
+                             const_cast<int*>(a->zero_counters), stream);
+  if (rc) return rc;
+  const double t_end = a->t + sec.dt;
+  int it = 0, n = a->guess < 1 ? 1 : a->guess;
+  for (;;) {
+    if (n > a->max_iterations - it) n = a->max_iterations - it;
+    const int first = it ? it + 1 : 0; /* iteration 0: the predictor's residual */
+    rc = prml_secant_run(a->secant_kernel, a->secant_tile[2], a->secant_tile[0], a->secant_tile[1], a->secant_box[0],
+                         a->secant_box[1], C, a->end, &sec, a->xa, a->xb, inst, t_end, first, it + n + 1 - first, stream);
+    if (rc) return rc;
+    it += n;
+    if (it >= a->max_iterations) break;
+    e = cudaMemcpyAsync(a->host_words, a->words, 4 * ints, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(PRML_ERR_CUDA, std::string("prml_secant_solve: ") + cudaGetErrorString(e));
+    bool all = true;
+    for (int b = 0; b < nb && all; ++b) {
+      const int* c = a->host_words + ((it % 3) * nb + b) * 2;
+      all = a->host_words[6 * nb + b] || !c[0] || !c[1];
+    }
+    if (all) break;
+    n = it / 2 > 8 ? it / 2 : 8;
+  }
+  rc = prml_secant_stop(a->ip, it, (it & 1) ? a->xa : a->xb, (it & 1) ? a->xb : a->xa, sec.flags, sec.counters, sec.done,
+                        it >= a->max_iterations, sec.res, sec.stats, stream);
+  if (rc) return rc;
+  rc = prml_implicit_finish(a->ip, sec.res, a->f0, a->out, stream);
+  if (rc) return rc;
+  e = cudaMemcpyAsync(a->host_words, a->words, bytes, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return fail(PRML_ERR_CUDA, std::string("prml_secant_solve: ") + cudaGetErrorString(e));
+  return PRML_OK;
 }
 
 }  // extern "C"

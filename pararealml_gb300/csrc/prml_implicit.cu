@@ -235,6 +235,43 @@ __global__ void mark_kernel(int batch, int* __restrict__ counters, int force, in
   if (threadIdx.x == 0) *iteration = it;
 }
 
+/* Finishes the instances still running after secant iteration k of the
+ * generated kernels (prml_secant_run): those that k stopped get the new
+ * iterate xn, with `force` the others the iterate before it, xp (the
+ * iteration limit).  Same results, flags and sums as the iteration that
+ * would follow. */
+__global__ void secant_stop_kernel(const prml_implicit_params p, int rows, long long n, int k,
+                                   const double* __restrict__ xn, const double* __restrict__ xp,
+                                   const unsigned char* __restrict__ flags, const int* __restrict__ counters,
+                                   int* done, int force, double* __restrict__ res, double* __restrict__ stats) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    Elem q;
+    if (!elem_of(p, e, rows, q)) continue;
+    const int d = *(volatile const int*)(done + q.b);
+    if (d && d < k) continue;
+    const int* c = counters + ((k % 3) * p.batch + q.b) * 2;
+    const bool flat = !c[0], stops = flat || !c[1];
+    if (!stops && !force) continue;
+    const unsigned char fl = flags[e];
+    double v = xp[e], other = xn[e];
+    if (stops) {
+      v = xn[e];
+      other = xp[e];
+      if (flat && !(fl & PRML_SECANT_MID)) v = __ddiv_rn(__dadd_rn(other, v), 2.0);
+    }
+    res[e] = v;
+    if (q.c == 0 && q.row == 0 && q.col == 0) *(volatile int*)(done + q.b) = k;
+    if (fl & PRML_SECANT_FAIL) {
+      atomicAdd(stats + 3 * q.b, 1.0);
+      if (!(fl & PRML_SECANT_NZ)) {
+        atomicAdd(stats + 3 * q.b + 1, 1.0);
+        const double diff = other - v;
+        if (other != v) atomicAdd(stats + 3 * q.b + 2, diff * diff);
+      }
+    }
+  }
+}
+
 int check(const prml_implicit_params* p) {
   if (!p) return prml_set_error(PRML_ERR_ARG, "implicit: null parameters");
   if (p->batch < 1 || p->comps < 1 || p->comps > 64 || p->pitch < p->n[2])
@@ -330,6 +367,19 @@ int prml_implicit_stop(const prml_implicit_params* p, const double* xs, const do
   if (rc) return rc;
   mark_kernel<<<1, IT, 0, s>>>(p->batch, counters, force ? 1 : 0, iteration, iterations);
   return last("implicit_stop(mark)");
+}
+
+int prml_secant_stop(const prml_implicit_params* p, int k, const double* xn, const double* xp,
+                     const unsigned char* flags, const int* counters, int* done, int force, double* res,
+                     double* stats, void* stream) {
+  int rc = check(p);
+  if (rc) return rc;
+  if (!xn || !xp || !flags || !counters || !done || !res || !stats || k < 1)
+    return prml_set_error(PRML_ERR_ARG, "secant_stop: bad argument");
+  const long long n = elems(p);
+  secant_stop_kernel<<<grid_of(n), IT, 0, static_cast<cudaStream_t>(stream)>>>(*p, rows_of(p), n, k, xn, xp, flags,
+                                                                              counters, done, force ? 1 : 0, res, stats);
+  return last("secant_stop");
 }
 
 int prml_implicit_finish(const prml_implicit_params* p, const double* x, const double* f, double* out,

@@ -171,8 +171,8 @@ def jacobi_coefficients(cs: str, d_x, axis_coords) -> np.ndarray:
 class StencilPlan:
     """Everything needed to launch fused FDM steps for one problem."""
 
-    # secant iterations an implicit step issues between two reads of the
-    # instances' finished counters
+    # secant iterations a run's first implicit step issues before it reads the
+    # instances' counters (later steps: as many as the step before took)
     IMPLICIT_BLOCK = 8
 
     def __init__(
@@ -564,33 +564,32 @@ class StencilPlan:
         # operator replaces them with its integrator's settings
         self.implicit = {"a": 0.5 if self.integrator == codegen.CRANK_NICOLSON else 1.0, "tol": 1.48e-8,
                          "max_iterations": 50, "crank_nicolson": self.integrator == codegen.CRANK_NICOLSON}
-        self._isec = self.new_state(8)  # p, p1, q0, q1, fu, f, result, f at the step start
+        # two iterates, residual, fu, result, right-hand side at the step start
+        self._isec = self.new_state(6)
         self._iflags = torch.empty(self.batch * self.inst, dtype=torch.uint8, device=self.device)
-        self._icount = torch.zeros((self.batch, 4), dtype=torch.int32, device=self.device)
-        self._istat = torch.zeros((self.batch, 4), dtype=torch.float64, device=self.device)
-        self._iits = torch.zeros(self.batch, dtype=torch.int32, device=self.device)
-        self._iiter = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self._implicit_stream = torch.cuda.Stream(device=self.device)
+        self._izero = torch.zeros((self.batch, 4), dtype=torch.int32, device=self.device)
+        # per step: counters [3][batch][2], done [batch] (ints), status sums
+        # [batch][3] (doubles), and their page-locked host copy
+        self._iblock = torch.zeros(14 * self.batch + 2, dtype=torch.int32, device=self.device)
+        self._ihost = torch.zeros_like(self._iblock, device="cpu").pin_memory()
+        self._iend = _native.StepParams()
 
     def _implicit_step(self, y: int, out: int, t: float, dt: float, slot_bytes: int, nb: int) -> None:
         """One backward Euler / Crank-Nicolson step from the device state at
         address ``y`` to ``out`` (numerical_integrator.py:199-270): forward
         Euler predictor, then the element-wise secant iteration of
         scipy.optimize.newton on the residual, every instance stopping on its
-        own.  The stop test, the result copy, the status sums and the
-        iteration count run on the device (``prml_implicit_stop``), and the
-        buffer roles repeat every two iterations, so two iterations are
-        recorded once per step as a CUDA graph and replayed; the host reads
-        the instances' finished counters every ``IMPLICIT_BLOCK`` iterations
-        (iterations of finished instances leave them unchanged) and raises
-        the reference's warnings and error from each instance's recorded
-        status, in the order the instances stopped.  ``self.params`` tables
-        point at the step start (half step 0)."""
+        own.  One launch of the generated secant kernel is one iteration
+        (right-hand side at the iterate, residual, secant step and the result
+        of the instances that the iteration before stopped), and one native
+        call issues the step: as many iterations as the previous step took,
+        then half as many again (at least 8) between two reads of the
+        counters (iterations of finished instances leave them unchanged).
+        The reference's warnings and error are raised from each instance's
+        recorded status, in the order the instances stopped.
+        ``self.params`` tables point at the step start (half step 0)."""
         import warnings
 
-        import torch
-
-        lib = _native.lib()
         ip = self._ip
         s = self.implicit
         ip.batch = nb
@@ -598,99 +597,46 @@ class StencilPlan:
         ip.a = s["a"]
         ip.tol = s["tol"]
         ip.crank_nicolson = int(s["crank_nicolson"])
-        base_dir, base_neu = self.params.dirichlet, self.params.neumann
-        ip.dirichlet = base_dir + 2 * slot_bytes  # constraints at t + dt
-        bufs = [self._isec[k].data_ptr() for k in range(4)]  # p, p1, q0, q1 (roles swap)
-        fu, f, f0 = self._isec[4].data_ptr(), self._isec[5].data_ptr(), self._isec[7].data_ptr()
-        res = self._isec[6].data_ptr()
-        cnt, stats, its_dev, counter = self._icount, self._istat, self._iits, self._iiter
-        flags = self._iflags.data_ptr()
+        ip.dirichlet = self.params.dirichlet + 2 * slot_bytes  # constraints at t + dt
+        gen = self.module.gen
+        rhs_name, rhs_smem, rhs_tile = gen.rhs_kernel
+        name, smem, tile = gen.secant_kernel
+        max_it = int(s["max_iterations"])
         batch_saved = self.params.batch
         self.params.batch = nb
-
-        def rhs_at(state, dst, when, slot):
-            self.params.dirichlet = base_dir + slot * slot_bytes
-            self.params.neumann = base_neu + slot * slot_bytes
-            self.rhs(state, dst, when)
-
-        def residual(xi, qi, prev):
-            rhs_at(bufs[xi], f, t + dt, 2)
-            _native.check(lib.prml_implicit_residual(
-                ctypes.byref(ip), bufs[xi], y, f, fu, bufs[qi], 0 if prev is None else bufs[prev],
-                cnt.data_ptr(), self.stream_handle()), "implicit residual")
-
-        def stop(xs, xo, force):
-            _native.check(lib.prml_implicit_stop(
-                ctypes.byref(ip), bufs[xs], bufs[xo], flags, cnt.data_ptr(), counter.data_ptr(), force, res,
-                stats.data_ptr(), its_dev.data_ptr(), self.stream_handle()), "implicit stop")
-
-        def iteration(roles, last):
-            """One secant iteration from the buffer roles (p, p1, q0, q1);
-            ``last``: the iteration limit, the instances still running stop
-            on the previous iterate.  Returns the next roles."""
-            p_, p1_, q0_, q1_ = roles
-            _native.check(lib.prml_implicit_update(
-                ctypes.byref(ip), bufs[p_], bufs[p1_], bufs[q0_], bufs[q1_], flags, cnt.data_ptr(),
-                self.stream_handle()), "implicit update")
-            stop(p_, p1_, 0)  # converged or flat: the new iterate
-            p_, p1_ = p1_, p_  # p1, p = p, p1
-            if last:
-                stop(p_, p1_, 1)  # exhausted: the previous iterate
-                return p_, p1_, q0_, q1_
-            q0_, q1_ = q1_, q0_  # q0 = q1; q1 <- the residual of the new p1
-            residual(p1_, q1_, q0_)
-            return p_, p1_, q0_, q1_
-
-        graph = None
         try:
-            cnt[:nb].zero_()
-            stats[:nb].zero_()
-            its_dev[:nb].zero_()
-            counter.zero_()
-            rhs_at(y, f0, t, 0)
-            _native.check(lib.prml_implicit_predict(
-                ctypes.byref(ip), y, f0, fu, bufs[0], bufs[1], flags, cnt.data_ptr(), self.stream_handle()),
-                "implicit predict")
-            residual(0, 2, None)
-            residual(1, 3, 2)
-            roles = (0, 1, 2, 3)
-            max_it = int(s["max_iterations"])
-            it, closed = 0, False
-            while it < max_it:
-                block_end = min(it + self.IMPLICIT_BLOCK, max_it)
-                while it < block_end:
-                    if block_end - it >= 2:
-                        if graph is None:
-                            # two iterations bring the roles back: record them
-                            # once, then replay (recording runs nothing)
-                            graph = torch.cuda.CUDAGraph()
-                            side = self._implicit_stream
-                            side.wait_stream(torch.cuda.current_stream())
-                            with torch.cuda.stream(side):
-                                graph.capture_begin(capture_error_mode="relaxed")
-                                try:
-                                    back = iteration(iteration(roles, False), False)
-                                finally:
-                                    graph.capture_end()
-                            torch.cuda.current_stream().wait_stream(side)
-                            assert back == roles
-                        graph.replay()
-                        it += 2
-                    else:
-                        it += 1
-                        closed = it == max_it
-                        roles = iteration(roles, closed)
-                if bool(cnt[:nb, 3].all()):
-                    break
-            if it == max_it and not closed:
-                stop(roles[0], roles[1], 1)  # the limit reached inside a replay
-            its = [int(v) for v in its_dev[:nb].cpu()]
-            stat = stats[:nb].cpu().numpy()
+            self.params.tile_z = max(1, codegen.tile_planes(rhs_tile))
+            self.params.jobs_per_cta = 1
+            self.params.box_planes = gen.box_depth(rhs_tile, mode=1)
+            end = self._iend  # the residuals read the boundary values at t + dt
+            ctypes.memmove(ctypes.byref(end), ctypes.byref(self.params), ctypes.sizeof(end))
+            end.dirichlet += 2 * slot_bytes
+            end.neumann += 2 * slot_bytes
+            end.tile_z = max(1, codegen.tile_planes(tile))
+            end.box_planes = gen.box_depth(tile, mode=1)
+            xa, xb, q, fu, res, f0 = (self._isec[k].data_ptr() for k in range(6))
+            last = self.secant_iterations[-1] if self.secant_iterations else None
+            step = _native.SecantStep(
+                rhs_kernel=self.module.kernel(rhs_name, rhs_smem), secant_kernel=self.module.kernel(name, smem),
+                rhs_tile=rhs_tile[:3], rhs_box=gen.box(rhs_tile, mode=1), secant_tile=tile[:3],
+                secant_box=gen.box(tile, mode=1), start=ctypes.pointer(self.params), end=ctypes.pointer(end),
+                ip=ctypes.pointer(ip),
+                sec=_native.SecantParams(y=y, fu=fu, q=q, flags=self._iflags.data_ptr(), res=res, a=ip.a, dt=ip.dt,
+                                         tol=ip.tol, crank_nicolson=ip.crank_nicolson),
+                xa=xa, xb=xb, f0=f0, out=out, words=self._iblock.data_ptr(), host_words=self._ihost.data_ptr(),
+                zero_counters=self._izero.data_ptr(), t=float(t), guess=max(last) + 1 if last else self.IMPLICIT_BLOCK,
+                max_iterations=max_it)
+            _native.check(_native.lib().prml_secant_solve(ctypes.byref(step), self.stream_handle()), "implicit step")
+            words = self._ihost.numpy()
+            its = [int(v) for v in words[6 * nb: 7 * nb]]
+            ints = 7 * nb + (nb & 1)
+            stat = words[ints: ints + 6 * nb].view(np.float64).reshape(nb, 3)
             self.secant_iterations.append(its)
+            n_all = self.C * self.nx * self.ny
             # numpy's post-loop checks (scipy.optimize.newton), instance by
             # instance in the order they stopped
             for b in sorted(range(nb), key=lambda b: (its[b], b)):
-                n_fail, n_all, n_zero, rms2 = stat[b]
+                n_fail, n_zero, rms2 = stat[b]
                 if n_zero > 0:
                     if rms2 > 0:
                         msg = f"RMS of {np.sqrt(rms2):g} reached"
@@ -703,11 +649,7 @@ class StencilPlan:
                         raise RuntimeError(msg)
                     self.secant_warnings.append(msg)
                     warnings.warn(msg, RuntimeWarning, stacklevel=5)
-            _native.check(lib.prml_implicit_finish(ctypes.byref(ip), res, f0, out, self.stream_handle()),
-                          "implicit finish")
         finally:
-            del graph
-            self.params.dirichlet, self.params.neumann = base_dir, base_neu
             self.params.batch = batch_saved
             ip.batch = self.batch
 
