@@ -69,6 +69,17 @@ int prml_fdm_run(void* kernel, int block, int tile_x, int tile_y, int box_rows, 
                  void* traj, long long traj_bstride, long long traj_step_stride,
                  void* work_a, void* work_b, long long work_bstride, long long n_steps,
                  int save_every, double t0, double dt, void* stream);
+/* prml_fdm_run for a stage kernel of a 3D module: one launch per integrator
+ * stage, each thread one 16-byte vector on `planes` planes.  stage_a and acc
+ * (more than one stage), stage_b (more than two): work states with instances
+ * work_bstride elements apart. */
+int prml_stage_params_size(void);
+int prml_fdm_run_stages(void* kernel, int block, int planes, const prml_step_params* base, int n_stages,
+                        const void* y0, long long y0_bstride, void* traj, long long traj_bstride,
+                        long long traj_step_stride, void* work_a, void* work_b, long long work_bstride, void* stage_a,
+                        void* stage_b, void* acc, long long n_steps, int save_every, double t0, double dt,
+                        void* stream);
+
 /* Evaluates the right-hand side of every equation at (t, y) into f
  * (reference: FDMSymbolMapper.map_concatenated, fdm_symbol_mapper.py:150-158). */
 int prml_fdm_rhs(void* kernel, int block, int tile_x, int tile_y, int box_rows, int box_cols,

@@ -143,6 +143,20 @@ typedef struct prml_multi_params {
   int n_rounds;          /* largest n_steps of the groups                    */
 } prml_multi_params;
 
+/* ---- one launch per integrator stage -------------------------------------
+ * Second parameter of the stage kernels: stage s of a multi-stage step reads
+ * its stencil input (stage 0: the state at the step start) and, element by
+ * element, the step's start and the slope sums, and writes the next stage's
+ * input (the last stage: the result) and the sums. */
+typedef struct prml_stage_params {
+  const void* y;         /* state at the step start                          */
+  long long y_bstride;   /* elements between its instances                   */
+  void* acc;             /* slope sums; planes of LHS.Y rows hold their value */
+  long long acc_bstride;
+  int stage;
+  int pad;
+} prml_stage_params;
+
 /* ---- secant iterations of an implicit step --------------------------------
  * One launch of a generated secant kernel (MODE 2 of the step body, float64)
  * is one iteration of the reference's element-wise secant solve: the

@@ -103,6 +103,9 @@ def _declare(lib: ctypes.CDLL) -> None:
             _c_int,
             [_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _p, _p, _c_ll, _p, _c_ll, _c_ll, _p, _p, _c_ll, _c_ll, _c_int, _c_d, _c_d, _p],
         ),
+        "prml_stage_params_size": (_c_int, []),
+        "prml_fdm_run_stages": (_c_int, [_p, _c_int, _c_int, _p, _c_int, _p, _c_ll, _p, _c_ll, _c_ll, _p, _p, _c_ll,
+                                         _p, _p, _p, _c_ll, _c_int, _c_d, _c_d, _p]),
         "prml_fdm_rhs": (_c_int, [_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _p, _p, _c_ll, _p, _c_ll, _c_d, _p]),
         "prml_set_step_overlap": (_c_int, [_c_int]),
         "prml_pack": (_c_int, [_p, _p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_int, _p]),
@@ -178,6 +181,8 @@ def exported_symbols() -> list:
         "prml_kernel_occupancy",
         "prml_fdm_run",
         "prml_fdm_rhs",
+        "prml_stage_params_size",
+        "prml_fdm_run_stages",
         "prml_set_step_overlap",
         "prml_pack",
         "prml_unpack",

@@ -22,6 +22,7 @@ from __future__ import annotations
 import dataclasses
 import functools
 import hashlib
+import re
 from typing import Dict, List, Sequence, Tuple
 
 import numpy as np
@@ -76,6 +77,11 @@ MARCH_JOBS: Tuple[int, ...] = (4, 8, 12, 16, 20, 24)
 # 2 / 2.5, 16 x 257^2 in float64 9.1 / 10.1 / 11.4 / 11.7 ms
 MARCH_EDGE = {4: 1.5, 8: 1.0}
 MARCH_THREADS = 128
+# 3D kernels launched once per integrator stage: planes per thread (97^3 RK4
+# in float64: 1, 2 and 4 planes 2.38, 2.54 and 2.64 ms per 20 steps; where a
+# step is bound by its reads more planes per thread read fewer rows)
+STAGE_PLANES: Tuple[int, ...] = (1, 2, 4)
+STAGE_THREADS = 128
 # 3D tiles (rows, cols, threads, 1, planes)
 TILE_CONFIGS_3D: Tuple[Tuple[int, int, int, int, int], ...] = (
     (8, 32, 256, 1, 2),
@@ -382,7 +388,7 @@ def _symbol_code(sym: sp.Symbol, low: LoweredProblem, fast: bool = False) -> str
         i = idx[0]
         for axis in range(x_dim):
             need3(axis)
-        if fast and x_dim == 2:
+        if fast and x_dim >= 2:
             return f"a.template lap<{i}>()"
         terms = [f"a.template sd<{i}, {ka[axis]}>()" for axis in range(x_dim)]
         return "(" + " + ".join(terms) + ")"
@@ -607,9 +613,14 @@ class _KernelPrinter(C99CodePrinter):
 
 
 def _folds_inv_dd(low: LoweredProblem, fast: bool) -> bool:
-    """Fused-order 2D Cartesian modules with equal steps along both axes
+    """Fused-order 2D and 3D Cartesian modules with equal steps along all axes
     write scaled Laplacians as lapr(y) * INV_DD."""
-    return fast and low.x_dimension == 2 and low.cs == "CARTESIAN" and low.dx_k[0] == low.dx_k[1]
+    return fast and low.x_dimension >= 2 and low.cs == "CARTESIAN" and _equal_steps(low)
+
+
+def _equal_steps(low: LoweredProblem) -> bool:
+    """Whether the mesh axes share one step size."""
+    return low.dx_k[0] == low.dx_k[1] and (low.x_dimension < 3 or low.dx_z == low.dx_k[0])
 
 
 def _rhs_function(name: str, rows: Sequence[int], low: LoweredProblem, fast: bool = False,
@@ -718,6 +729,11 @@ def is_walk(tile) -> bool:
     return len(tile) > 5 and tile[5] == "w"
 
 
+def is_stage(tile) -> bool:
+    """Whether a tile key names a kernel launched once per integrator stage."""
+    return len(tile) > 5 and tile[5] == "s"
+
+
 def is_march(tile) -> bool:
     """Whether a tile key names a marching kernel (march_body)."""
     return len(tile) > 5 and tile[5] == "m"
@@ -766,6 +782,8 @@ def walk_tile(rows_per_thread: int, warps: int, esize: int) -> tuple:
 def kernel_name(kind: str, dtype: str, tile) -> str:
     if is_march(tile):
         return f"prml_march_{dtype}_v{tile[6]}" + (f"_k{tile[3]}" if tile[3] > 1 else "")
+    if is_stage(tile):
+        return f"prml_stage_{dtype}_z{tile[4]}"
     if is_walk(tile):
         return f"prml_walk_{dtype}_{tile[0]}x{tile[1]}x{tile[2]}"
     if tile_planes(tile):
@@ -834,18 +852,20 @@ class GeneratedModule:
     multi_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
     # secant-iteration kernel of modules with exact division: (name, smem, tile)
     secant_kernel: Tuple[str, int, tuple] = None
+    # 3D kernels launched once per integrator stage: tile (1, cols, threads, 1, planes, "s") -> (name, smem)
+    stage_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
     # marching kernels: tile (jobs per SM, cols, threads, steps, 0, "m", columns per lane) -> (name, smem)
     march_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
 
     @functools.cached_property
     def kernels(self) -> Dict[tuple, Tuple[str, int]]:
         """Every step kernel: tile -> (name, dynamic shared memory)."""
-        return {**self.step_kernels, **self.march_kernels}
+        return {**self.step_kernels, **self.march_kernels, **self.stage_kernels}
 
     def box(self, tile, mode: int = 0) -> Tuple[int, int]:
         """TMA box (rows, cols) a kernel of this module stages."""
         esize = 8 if self.dtype == "f64" else 4
-        if is_march(tile):  # no tile is staged: any box the tensor map accepts
+        if is_march(tile) or is_stage(tile):  # no tile is staged: any box the tensor map accepts
             return 1, 16 // esize
         return region(tile, halo(self.integrator, self.invariant, mode, tile), esize)
 
@@ -855,7 +875,7 @@ class GeneratedModule:
 
     def box_depth(self, tile, mode: int = 0) -> int:
         """Mesh planes of the TMA box of a 3D kernel (1 for 2D kernels)."""
-        if not tile_planes(tile):
+        if not tile_planes(tile) or is_stage(tile):
             return 1
         return tile_planes(tile) + 2 * halo(self.integrator, self.invariant, mode, tile)
 
@@ -870,10 +890,10 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
     into differences of the order of its tolerance) instead of multiplying
     by reciprocals.
 
-    ``fast`` (fused operation order; 1D and 2D meshes, not with
-    ``exact_div``): the Cartesian Laplacian is one neighbour sum minus four
-    (two per axis) times the centre, scaled once; sums with a product term
-    are multiply-adds; the integrator combines unscaled slopes and scales
+    ``fast`` (fused operation order; not with ``exact_div``): the Cartesian
+    Laplacian is one neighbour sum minus four times the centre (2D) or the sum
+    of the second differences (3D), scaled once; sums with a product term are
+    multiply-adds; the integrator combines unscaled slopes and scales
     them once (a stage-invariant RK4 step is y + dt f).  Each result stays
     within a few roundings of the reference's operation order, with about
     half the floating-point operations per vertex (the float64 pipe of this
@@ -883,7 +903,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
     step of several groups of instances in one cooperative launch)."""
     if integrator not in (FORWARD_EULER, EXPLICIT_MIDPOINT, RK4):
         raise ValueError(f"unsupported integrator {integrator}")
-    fast = bool(fast) and not exact_div and low.x_dimension != 3
+    fast = bool(fast) and not exact_div
     ctype = {"f32": "float", "f32c": "float", "f64": "double"}[dtype]
     esize = 8 if dtype == "f64" else 4
     comp = 1 if dtype == "f32c" else 0
@@ -892,6 +912,8 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
     uses_t = any(sym.name == "t" for expr in low.rhs for sym in expr.free_symbols)
     d_rows, y_rows = list(low.d_idx), list(low.y_idx)
     side_mask, corners = _side_columns(low)
+    rhs_code = [_rhs_function("rhs_dt", d_rows, low, fast), _rhs_function("rhs_y", y_rows, low, fast)]
+    corners = corners or any(a != b for a, b in re.findall(r"hess<\d+, (\d), (\d)>", "".join(rhs_code)))
     three_d = low.x_dimension == 3
     if three_d and comp:
         raise NotImplementedError("compensated float32 is not available on 3D meshes")
@@ -906,7 +928,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         f"  static constexpr bool USES_T = {'true' if uses_t else 'false'};",
         f"  static constexpr bool EXACT_DIV = {'true' if exact_div else 'false'};",
         f"  static constexpr bool FAST = {'true' if fast else 'false'};",
-        f"  static constexpr bool EQUAL_DX = {'true' if low.dx_k[0] == low.dx_k[1] else 'false'};",
+        f"  static constexpr bool EQUAL_DX = {'true' if _equal_steps(low) else 'false'};",
         f"  static constexpr unsigned HMASK = {side_mask}u;",
         f"  static constexpr bool CORNERS = {'true' if corners else 'false'};",
         f"  static constexpr bool DYNAMIC = {'true' if low.dynamic else 'false'};",
@@ -917,8 +939,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         f"  static constexpr unsigned long long DIR_MASK = {low.dir_mask}ull;",
         f"  static __device__ constexpr int dcomp(int i) {{ return {_chain(d_rows)}; }}",
         f"  static __device__ constexpr int ycomp(int i) {{ return {_chain(y_rows)}; }}",
-        _rhs_function("rhs_dt", d_rows, low, fast),
-        _rhs_function("rhs_y", y_rows, low, fast),
+        *rhs_code,
         _rhs_function("rhs_dt_split", d_rows, low, fast, split=True) if fast else "",
         "};",
         "",
@@ -948,6 +969,17 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
             f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin) "
             f"{{ prml::step_body3<{ctype}, Eq, {integrator}, {rtile[4]}, {rtile[0]}, {rtile[1]}, {rtile[2]}, 1>(p, tin); }}"
         )
+        stage_kernels = {}
+        if not invariant and not low.lap_idx and not exact_div:
+            for planes in STAGE_PLANES:
+                tile = (1, 16 // esize, STAGE_THREADS, 1, planes, "s")
+                name = kernel_name("stage", dtype, tile)
+                stage_kernels[tile] = (name, 0)
+                body.append(
+                    f'extern "C" __global__ void __launch_bounds__({STAGE_THREADS}) {name}'
+                    f"(const prml_step_params p, const prml_stage_params s) "
+                    f"{{ prml::stage_body3<{ctype}, Eq, {integrator}, {planes}, {STAGE_THREADS}>(p, s); }}"
+                )
         secant = None
         if exact_div and ctype == "double":
             sname = kernel_name("secant", dtype, rtile)
@@ -962,7 +994,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         key = hashlib.sha256((source + _template_digest()).encode()).hexdigest()[:24]
         return GeneratedModule(source=source, key=key, dtype=dtype, integrator=integrator, invariant=invariant,
                                step_kernels=step_kernels, rhs_kernel=(rname, rsm, rtile), n_comp=low.n_comp,
-                               secant_kernel=secant)
+                               secant_kernel=secant, stage_kernels=stage_kernels)
     # temporally blocked kernels take several steps per launch; a Jacobi
     # solve has to run between every two steps
     blocked = single_stage and not low.lap_idx

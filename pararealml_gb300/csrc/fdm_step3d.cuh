@@ -89,21 +89,51 @@ struct Point3 {
   }
   template <int c, int ka> __device__ __forceinline__ T grad() const { return grad_at<c, ka, false>(0, 0, 0); }
 
-  /* second derivative along kernel axis ka with Neumann ghost vertices */
-  template <int c, int ka> __device__ __forceinline__ T sd() const {
+  /* neighbours (prev, next) along kernel axis ka with Neumann ghost vertices */
+  template <int c, int ka> __device__ __forceinline__ void ends(T& prev, T& next) const {
     const int e0 = ka == 0, e1 = ka == 1, e2 = ka == 2;
-    const T lo = v(c, -e0, -e1, -e2), hi = v(c, e0, e1, e2), mid = v(c, 0, 0, 0);
-    T prev = lo, next = hi;
+    const T lo = v(c, -e0, -e1, -e2), hi = v(c, e0, e1, e2);
+    prev = lo;
+    next = hi;
     if (has_neu(2 * ka, c) && g[ka] == 0) {
       const T gv = face(m->neu, 2 * ka, c, g[0], g[1], g[2]);
-      if (gv == gv) prev = hi - m->twod[ka] * gv;
+      if (gv == gv) prev = Eq::FAST ? fmaT(-m->twod[ka], gv, hi) : hi - m->twod[ka] * gv;
     }
     if (has_neu(2 * ka + 1, c) && g[ka] == m->n[ka] - 1) {
       const T gv = face(m->neu, 2 * ka + 1, c, g[0], g[1], g[2]);
-      if (gv == gv) next = lo + m->twod[ka] * gv;
+      if (gv == gv) next = Eq::FAST ? fmaT(m->twod[ka], gv, lo) : lo + m->twod[ka] * gv;
     }
+  }
+
+  /* second derivative along kernel axis ka */
+  template <int c, int ka> __device__ __forceinline__ T sd() const {
+    const T mid = v(c, 0, 0, 0);
+    T prev, next;
+    ends<c, ka>(prev, next);
     if constexpr (Eq::EXACT_DIV) return quot(fmaT(T(-2), mid, next) + prev, m->dd[ka], m->invdd[ka]);
     return ((next - T(2) * mid) + prev) * m->invdd[ka];
+  }
+
+  /* second difference along kernel axis ka, unscaled: (next - 2 y) + prev as
+   * in sd (2 y is exact, so one multiply-add rounds like the product and the
+   * difference) */
+  template <int c, int ka> __device__ __forceinline__ T dd() const {
+    T prev, next;
+    ends<c, ka>(prev, next);
+    return fmaT(T(-2), v(c, 0, 0, 0), next) + prev;
+  }
+
+  /* Laplacian in fused order: the second differences of sd summed before one
+   * scaling (lapr: unscaled, for a term that carries inv_dd()) where all axes
+   * share a step size, scaled by multiply-adds otherwise.  Not the neighbour
+   * sum of the 2D kernels: two operations less, but six neighbours summed
+   * first round at six times the vertex's size and the error of a step grows
+   * (8e-17 against 1e-17 of a float64 state after 20 steps). */
+  template <int c> __device__ __forceinline__ T lapr() const { return (dd<c, 0>() + dd<c, 1>()) + dd<c, 2>(); }
+  __device__ __forceinline__ T inv_dd() const { return m->invdd[0]; }
+  template <int c> __device__ __forceinline__ T lap() const {
+    if constexpr (Eq::EQUAL_DX) return lapr<c>() * m->invdd[0];
+    return fmaT(dd<c, 0>(), m->invdd[0], fmaT(dd<c, 1>(), m->invdd[1], dd<c, 2>() * m->invdd[2]));
   }
 
   /* Hessian element (kernel axes a1, a2): d/d a2 of the constrained d/d a1 */
@@ -137,6 +167,45 @@ __device__ __forceinline__ MeshC3<T> mesh3_at(const MeshC3<T>& m, const prml_ste
   r.dir = m.dir + off;
   r.neu = m.neu + off;
   return r;
+}
+
+/* mesh constants, tables and coordinates in kernel axis order */
+template <typename T>
+__device__ __forceinline__ MeshC3<T> mesh3_of(const prml_step_params& p) {
+  MeshC3<T> m;
+  const double i2[3] = {p.inv_2dx2, p.inv_2dx0, p.inv_2dx1};
+  const double idd[3] = {p.inv_dxx2, p.inv_dxx0, p.inv_dxx1};
+  const double tw[3] = {p.two_dx2, p.two_dx0, p.two_dx1};
+  const float i2f[3] = {p.inv_2dx2_f, p.inv_2dx0_f, p.inv_2dx1_f};
+  const float iddf[3] = {p.inv_dxx2_f, p.inv_dxx0_f, p.inv_dxx1_f};
+  const float twf[3] = {p.two_dx2_f, p.two_dx0_f, p.two_dx1_f};
+  const double ddd[3] = {p.dxx2, p.dxx0, p.dxx1};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if constexpr (sizeof(T) == 4) {
+      m.inv2d[a] = i2f[a];
+      m.invdd[a] = iddf[a];
+      m.twod[a] = twf[a];
+    } else {
+      m.inv2d[a] = T(i2[a]);
+      m.invdd[a] = T(idd[a]);
+      m.twod[a] = T(tw[a]);
+    }
+    m.dd[a] = T(ddd[a]);
+  }
+  m.n[0] = p.nz;
+  m.n[1] = p.nx;
+  m.n[2] = p.ny;
+  m.flen = p.face_len;
+  m.dir = static_cast<const T*>(p.dirichlet);
+  m.neu = static_cast<const T*>(p.neumann);
+  m.c[0] = p.coord2;
+  m.c[1] = p.coord0;
+  m.c[2] = p.coord1;
+  m.cf[0] = p.coord2_f;
+  m.cf[1] = p.coord0_f;
+  m.cf[2] = p.coord1_f;
+  return m;
 }
 
 /* 5D TMA box (cols, rows, planes, components, instance x slot) */
@@ -250,31 +319,14 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
           T v = y;
 #pragma unroll
           for (int i = 0; i < ND; ++i) {
-            if (Eq::dcomp(i) == c) {
-              if (INTEG == RK4) {
-                const T k = dt * f[i];
-                v = (s == 2) ? y + k : y + k * T(0.5);
-              } else {
-                v = y + (dt * T(0.5)) * f[i];
-              }
-            }
+            if (Eq::dcomp(i) == c) v = stage_input<T, Eq, INTEG>(y, f[i], dt, s);
           }
           nxt[c * RV + l] = dirichlet3<T, Eq>(v, c, g, mn);
         }
       }
       if (q >= 0) {
 #pragma unroll
-        for (int i = 0; i < ND; ++i) {
-          if (INTEG == RK4) {
-            const T k = dt * f[i];
-            if (Eq::STAGE_INVARIANT) acc[q][i] = ((k + T(2) * k) + T(2) * k) + k;
-            else if (s == 0) acc[q][i] = k;
-            else if (s == 3) acc[q][i] = acc[q][i] + k;
-            else acc[q][i] = acc[q][i] + T(2) * k;
-          } else {
-            acc[q][i] = dt * f[i];
-          }
-        }
+        for (int i = 0; i < ND; ++i) stage_accumulate<T, Eq, INTEG>(acc[q][i], f[i], dt, s);
       }
     };
 
@@ -315,6 +367,9 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
    * Dirichlet at t + dt, store */
   const MeshC3<T> m0 = mesh3_at(m, p, bc_slot(p, b));
   const MeshC3<T> m2 = mesh3_at(m, p, bc_slot(p, b) + 2);
+  /* fused order: the accumulated slopes' scale (RK4 of several stages: dt / 6) */
+  const T acc_scale = INTEG == RK4 && !Eq::STAGE_INVARIANT ? dt * T(1.0 / 6.0) : dt;
+  (void)acc_scale;
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
     const int k = threadIdx.x + q * NT;
@@ -335,7 +390,7 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
       T v = y;
 #pragma unroll
       for (int i = 0; i < ND; ++i)
-        if (Eq::dcomp(i) == c) v = (INTEG == RK4) ? y + div6(acc[q][i]) : y + acc[q][i];
+        if (Eq::dcomp(i) == c) v = step_result<T, Eq, INTEG>(y, acc[q][i], acc_scale);
 #pragma unroll
       for (int i = 0; i < Eq::NYC; ++i)
         if (Eq::ycomp(i) == c) v = yrhs[i];
@@ -375,39 +430,7 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
   const int per_inst = tiles_c * tiles_r * tiles_p;
   const int total = per_inst * p.batch;
 
-  MeshC3<T> m;
-  const double i2[3] = {p.inv_2dx2, p.inv_2dx0, p.inv_2dx1};
-  const double idd[3] = {p.inv_dxx2, p.inv_dxx0, p.inv_dxx1};
-  const double tw[3] = {p.two_dx2, p.two_dx0, p.two_dx1};
-  const float i2f[3] = {p.inv_2dx2_f, p.inv_2dx0_f, p.inv_2dx1_f};
-  const float iddf[3] = {p.inv_dxx2_f, p.inv_dxx0_f, p.inv_dxx1_f};
-  const float twf[3] = {p.two_dx2_f, p.two_dx0_f, p.two_dx1_f};
-  const double ddd[3] = {p.dxx2, p.dxx0, p.dxx1};
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    if constexpr (sizeof(T) == 4) {
-      m.inv2d[a] = i2f[a];
-      m.invdd[a] = iddf[a];
-      m.twod[a] = twf[a];
-    } else {
-      m.inv2d[a] = T(i2[a]);
-      m.invdd[a] = T(idd[a]);
-      m.twod[a] = T(tw[a]);
-    }
-    m.dd[a] = T(ddd[a]);
-  }
-  m.n[0] = p.nz;
-  m.n[1] = p.nx;
-  m.n[2] = p.ny;
-  m.flen = p.face_len;
-  m.dir = static_cast<const T*>(p.dirichlet);
-  m.neu = static_cast<const T*>(p.neumann);
-  m.c[0] = p.coord2;
-  m.c[1] = p.coord0;
-  m.c[2] = p.coord1;
-  m.cf[0] = p.coord2_f;
-  m.cf[1] = p.coord0_f;
-  m.cf[2] = p.coord1_f;
+  const MeshC3<T> m = mesh3_of<T>(p);
 
   auto coords = [&](int t, int& b, int& tz, int& ty, int& tx) {
     b = t / per_inst;
@@ -453,6 +476,193 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
     tile_compute3<T, Eq, INTEG, TZ, TX, TY, NT, MODE>(p, m, buf ? ybuf1 : ybuf0, bufA, bufB, b, tz * TZ,
                                                      ty * TX, tx * TY, sec);
     __syncthreads();
+  }
+}
+
+/* One integrator stage per launch (prml_stage_params): a thread holds 16 bytes
+ * of columns on Z planes of one row, its window read straight into registers.
+ * No staging, no shared memory, no barrier.
+ *
+ * Why: a whole RK4 step on a staged tile needs a halo of four vertices on
+ * every side, and the shells around a 2 x 8 x 32 tile are several times the
+ * tile over the four stages, all through the float64 pipe or the issue slots.
+ * One launch per stage recomputes nothing, for 17 state-sized reads and writes
+ * per step instead of two, from L2 where the states fit.
+ * GB300, us per RK4 step, the best staged whole-step tile against this (both
+ * fused order): 13^3 vertices 31 -> 17 in float64 and 16.5 -> 15.5 in float32,
+ * 49^3 136 -> 45 and 36 -> 18, 97^3 723 -> 126 and 148 -> 26 (before the
+ * fused order 967 in float64).  What bounds it: 97^3 in float64 the float64
+ * pipe (about 15 instructions a vertex and stage with the faces', 22 us of
+ * 33), small meshes the four dependent launches.  One-stage steps: 49^3
+ * 4.6 -> 3.9 and 97^3 10.9 -> 6.1 in float32, 97^3 34 -> 31 in float64; 13^3
+ * 3.5 -> 3.8 (the tuner keeps the staged tile there).
+ *
+ * Work: the vectors of a plane chunk in row order, one per thread, so that
+ * only the last warp of an instance is partly empty (an 8-lane group per row
+ * segment, as on 2D meshes, leaves a fifth of the lanes idle on 97 columns).
+ * The neighbouring columns come from the neighbouring lanes; the first and
+ * last lane of the warp read theirs. */
+template <typename T, class Eq, int INTEG, int Z, int NT>
+__device__ __forceinline__ void stage_body3(const prml_step_params& p, const prml_stage_params& sp) {
+  constexpr int C = Eq::C;
+  constexpr int ND = Eq::ND;
+  constexpr int VW = 16 / (int)sizeof(T);
+  constexpr int NC = VW + 2, NRC = 3 * NC, NV = (Z + 2) * NRC;
+  static_assert(!Eq::STAGE_INVARIANT, "stage-invariant steps take one launch of the whole-step kernels");
+  using P = Point3<T, Eq, NC, NRC, NV>;
+
+  const MeshC3<T> m = mesh3_of<T>(p);
+  const unsigned vecs = (unsigned)(p.ny + VW - 1) / VW;
+  const unsigned jobs = (unsigned)((p.nz + Z - 1) / Z) * (unsigned)p.nx * vecs;
+  const unsigned blocks = (jobs + NT - 1) / NT;
+  const unsigned b = blockIdx.x / blocks;
+  unsigned job = (blockIdx.x - b * blocks) * NT + threadIdx.x;
+  const bool active = job < jobs;
+  if (!active) job = jobs - 1; /* takes part in the shuffles, stores nothing */
+  const unsigned line = job / vecs;
+  const int gj0 = (int)(job - line * vecs) * VW;
+  const unsigned chunk = line / (unsigned)p.nx;
+  const int gi = (int)(line - chunk * p.nx);
+  const int gk0 = (int)chunk * Z;
+  const int lane = threadIdx.x & 31;
+
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  const long long plane = (long long)p.nx * p.pitch;
+  const long long o = gk0 * plane + (long long)gi * p.pitch + gj0;
+  const T* in = static_cast<const T*>(p.in) + (long long)b * p.in_bstride + o;
+  T* out = static_cast<T*>(p.out) + (long long)b * p.out_bstride + o;
+  const T* yg = static_cast<const T*>(sp.y) + (long long)b * sp.y_bstride + o;
+  T* ag = static_cast<T*>(sp.acc) + (long long)b * sp.acc_bstride + o;
+  const int s = sp.stage;
+  const bool first = s == 0, last = s == INTEG - 1;
+
+  /* planes gk0 - 1 .. gk0 + Z, rows gi - 1 .. gi + 1, columns gj0 - 1 .. gj0 +
+   * VW, zero outside the mesh; what no derivative reads is not loaded */
+  T w[C * NV];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+#pragma unroll
+    for (int z = -1; z <= Z; ++z) {
+#pragma unroll
+      for (int r = -1; r <= 1; ++r) {
+        const bool own = z >= 0 && z < Z && r == 0;
+        const bool star = r == 0 || (z >= 0 && z < Z);
+        if (!own && !((Eq::HMASK >> c) & 1u && (star || Eq::CORNERS))) continue;
+        T* row = w + c * NV + (z + 1) * NRC + (r + 1) * NC;
+        if (gk0 + z >= 0 && gk0 + z < p.nz && gi + r >= 0 && gi + r < p.nx) {
+          ld16(in + c * p.cstride + z * plane + r * p.pitch, row + 1);
+        } else {
+#pragma unroll
+          for (int k = 0; k < VW; ++k) row[1 + k] = T(0);
+        }
+      }
+    }
+  }
+  T y[Z][C][VW], a[Z][C][VW];
+#pragma unroll
+  for (int z = 0; z < Z; ++z) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+#pragma unroll
+      for (int k = 0; k < VW; ++k) {
+        y[z][c][k] = w[c * NV + (z + 1) * NRC + NC + 1 + k];
+        a[z][c][k] = T(0);
+      }
+      if (!first && gk0 + z < p.nz) {
+        ld16(yg + c * p.cstride + z * plane, y[z][c]);
+        ld16(ag + c * p.cstride + z * plane, a[z][c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    if (!((Eq::HMASK >> c) & 1u)) continue;
+#pragma unroll
+    for (int z = -1; z <= Z; ++z) {
+#pragma unroll
+      for (int r = -1; r <= 1; ++r) {
+        const bool own = z >= 0 && z < Z && r == 0;
+        const bool star = r == 0 || (z >= 0 && z < Z);
+        if (!star && !Eq::CORNERS) continue;
+        T* row = w + c * NV + (z + 1) * NRC + (r + 1) * NC;
+        /* the row padding holds no state */
+#pragma unroll
+        for (int k = 1; k < VW; ++k)
+          if (gj0 + k >= p.ny) row[1 + k] = T(0);
+        if (!own && !Eq::CORNERS) continue;
+        T left = __shfl_up_sync(0xffffffffu, row[VW], 1);
+        T right = __shfl_down_sync(0xffffffffu, row[1], 1);
+        const bool in_mesh = gk0 + z >= 0 && gk0 + z < p.nz && gi + r >= 0 && gi + r < p.nx;
+        const T* src = in + c * p.cstride + z * plane + r * p.pitch;
+        if (lane == 0 && gj0 > 0 && in_mesh) left = __ldcg(src - 1);
+        if (lane == 31 && gj0 + VW < p.ny && in_mesh) right = __ldcg(src + VW);
+        row[0] = gj0 > 0 && in_mesh ? left : T(0);
+        row[NC - 1] = gj0 + VW < p.ny && in_mesh ? right : T(0);
+      }
+    }
+  }
+  if (!active) return;
+
+  const double ts = Eq::USES_T ? p.t + (p.t_offset ? p.t_offset[b] : 0.0) + stage_time<INTEG>(s) * p.dt : 0.0;
+  const T dt = step_dt<T>(p);
+  const T acc_scale = INTEG == RK4 ? dt * T(1.0 / 6.0) : dt;
+  const int slot0 = bc_slot(p, b);
+  const MeshC3<T> ms = mesh3_at(m, p, slot0 + stage_half<INTEG>(s));
+  const MeshC3<T> me = mesh3_at(m, p, slot0 + (last ? 2 : stage_half<INTEG>(s + 1)));
+#pragma unroll
+  for (int z = 0; z < Z; ++z) {
+    if (gk0 + z >= p.nz) break;
+    T res[C][VW];
+#pragma unroll
+    for (int k = 0; k < VW; ++k) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) res[c][k] = T(0);
+      if (gj0 + k >= p.ny) continue;
+      const int g[3] = {gk0 + z, gi, gj0 + k};
+      P pt{w, (z + 1) * NRC + NC + 1 + k, {g[0], g[1], g[2]}, &ms, ts};
+      T f[ND > 0 ? ND : 1];
+      if (ND > 0) Eq::rhs_dt(pt, f);
+      T yrhs[Eq::NYC > 0 ? Eq::NYC : 1];
+      if (Eq::NYC > 0 && first) Eq::rhs_y(pt, yrhs);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        T v = y[z][c][k];
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+          if (Eq::dcomp(i) == c) {
+            stage_accumulate<T, Eq, INTEG>(a[z][c][k], f[i], dt, s);
+            v = last ? step_result<T, Eq, INTEG>(y[z][c][k], a[z][c][k], acc_scale)
+                     : stage_input<T, Eq, INTEG>(y[z][c][k], f[i], dt, s);
+          }
+        }
+        /* LHS.Y rows: their value at the step start, kept in the sums' plane */
+#pragma unroll
+        for (int i = 0; i < Eq::NYC; ++i) {
+          if (Eq::ycomp(i) == c) {
+            if (first) a[z][c][k] = yrhs[i];
+            if (last) v = a[z][c][k];
+          }
+        }
+        res[c][k] = dirichlet3<T, Eq>(v, c, g, me);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const long long e = c * p.cstride + z * plane;
+      if (gj0 + VW <= p.ny) {
+        st16(out + e, res[c]);
+        if (!last) st16(ag + e, a[z][c]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < VW; ++k) {
+          if (gj0 + k >= p.ny) break;
+          out[e + k] = res[c][k];
+          if (!last) ag[e + k] = a[z][c][k];
+        }
+      }
+    }
   }
 }
 

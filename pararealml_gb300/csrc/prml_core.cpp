@@ -416,9 +416,9 @@ int prml_set_step_overlap(int enabled) {
   return prev;
 }
 
-static int launch_step(Kernel* k, int block, int grid, prml_step_params* p, CUtensorMap* map,
-                       CUstream stream, prml_secant_params* sec = nullptr) {
-  void* args[] = {p, map, sec};
+static int launch_step(Kernel* k, int block, int grid, prml_step_params* p, void* second,
+                       CUstream stream, void* third = nullptr) {
+  void* args[] = {p, second, third};
   CUresult r;
   if (g_step_overlap && g_drv.LaunchKernelEx) {
     CUlaunchAttribute attr[1];
@@ -548,6 +548,76 @@ int prml_fdm_run(void* kernel, int block, int tile_x, int tile_y, int box_rows, 
     cur_bstride = out_bstride;
     cur_map = out_map;
     cur_slot = out_slot;
+  }
+  return PRML_OK;
+}
+
+int prml_stage_params_size(void) { return (int)sizeof(prml_stage_params); }
+
+int prml_fdm_run_stages(void* kernel, int block, int planes, const prml_step_params* base, int n_stages,
+                        const void* y0, long long y0_bstride, void* traj, long long traj_bstride,
+                        long long traj_step_stride, void* work_a, void* work_b, long long work_bstride, void* stage_a,
+                        void* stage_b, void* acc, long long n_steps, int save_every, double t0, double dt,
+                        void* stream) {
+  Kernel* k = static_cast<Kernel*>(kernel);
+  if (!k) return fail(PRML_ERR_ARG, "prml_fdm_run_stages: null kernel");
+  if (!base) return fail(PRML_ERR_ARG, "null params");
+  int rc = check_geometry(base, base->nx < 1 ? 1 : base->nx, 1, block);
+  if (rc) return rc;
+  if (!y0 || !traj || n_steps < 0 || save_every < 1 || planes < 1 || base->nz < 1 || n_stages < 1 || n_stages > 4 ||
+      (n_stages > 1 && (!stage_a || !acc)) || (n_stages > 2 && !stage_b))
+    return fail(PRML_ERR_ARG, "prml_fdm_run_stages: bad buffers, stage or step counts");
+  if (n_steps % save_every != 0)
+    return fail(PRML_ERR_ARG, "prml_fdm_run_stages: n_steps must be a multiple of save_every");
+  if (save_every > 1 && (!work_a || !work_b))
+    return fail(PRML_ERR_ARG, "prml_fdm_run_stages: strided output needs two work buffers");
+  if (n_steps == 0) return PRML_OK;
+  /* one vector of 16 bytes times `planes` planes per thread (stage_body3) */
+  const int vw = 16 / base->elem_bytes;
+  const long long jobs = (long long)((base->nz + planes - 1) / planes) * base->nx * ((base->ny + vw - 1) / vw);
+  const long long blocks = (jobs + block - 1) / block * base->batch;
+  if (jobs + block >= (1LL << 31) || blocks >= (1LL << 31))
+    return fail(PRML_ERR_ARG, "too many tiles for one launch (2^31)");
+  const int grid = (int)blocks;
+  const size_t ebytes = (size_t)base->elem_bytes;
+  prml_step_params p = *base;
+  p.tb_steps = 1;
+  p.dt = dt;
+  p.dt_f = (float)dt;
+  prml_stage_params sp;
+  std::memset(&sp, 0, sizeof(sp));
+  sp.acc = acc;
+  sp.acc_bstride = work_bstride;
+  const char* cur = static_cast<const char*>(y0);
+  long long cur_bstride = y0_bstride;
+  int ping = 0;
+  for (long long step = 1; step <= n_steps; ++step) {
+    char* out;
+    long long out_bstride;
+    if (step % save_every == 0) {
+      out = static_cast<char*>(traj) + (size_t)(step / save_every - 1) * traj_step_stride * ebytes;
+      out_bstride = traj_bstride;
+    } else {
+      out = static_cast<char*>(ping ? work_b : work_a);
+      ping ^= 1;
+      out_bstride = work_bstride;
+    }
+    sp.y = cur;
+    sp.y_bstride = cur_bstride;
+    p.t = t0 + (double)(step - 1) * dt;
+    p.bc_slot0 = base->bc_slot0 + (int)(2 * (step - 1));
+    for (int s = 0; s < n_stages; ++s) {
+      const bool last = s == n_stages - 1;
+      sp.stage = s;
+      p.in = s == 0 ? cur : static_cast<const char*>((s & 1) ? stage_a : stage_b);
+      p.in_bstride = s == 0 ? cur_bstride : work_bstride;
+      p.out = last ? out : static_cast<char*>((s & 1) ? stage_b : stage_a);
+      p.out_bstride = last ? out_bstride : work_bstride;
+      rc = launch_step(k, block, grid, &p, &sp, static_cast<CUstream>(stream));
+      if (rc) return rc;
+    }
+    cur = out;
+    cur_bstride = out_bstride;
   }
   return PRML_OK;
 }

@@ -168,6 +168,11 @@ def jacobi_coefficients(cs: str, d_x, axis_coords) -> np.ndarray:
     return np.concatenate([1.0 / (2.0 * d_x[0] * r), 1.0 / r_sqr, 1.0 / step])
 
 
+# Most device memory a run takes for the stage inputs and slope sums of kernels
+# launched once per integrator stage; larger states keep the whole-step kernels.
+STAGE_WORK_BYTES = 8 << 30
+
+
 class StencilPlan:
     """Everything needed to launch fused FDM steps for one problem."""
 
@@ -843,14 +848,15 @@ class StencilPlan:
 
     def _launch(self, tile, y0, y0_bstride, traj, traj_bstride, traj_step_stride, wa, wb,
                 n_steps, save_every, t0, dt) -> None:
-        if codegen.is_walk(tile) or codegen.is_march(tile):
+        stage = codegen.is_stage(tile)
+        if codegen.is_walk(tile) or codegen.is_march(tile) or stage:
             # these kernels move up to 16 bytes per access: every buffer,
             # instance and step must start on a 16-byte boundary
             vw = 16 // self.esize
             strides = (y0_bstride, traj_bstride, traj_step_stride, self.inst)
             addrs = [a for a in (y0, traj, wa, wb) if a]
             if any(a % 16 for a in addrs) or any(s % vw for s in strides):
-                raise ValueError("register-window and marching step kernels need 16-byte aligned states and strides")
+                raise ValueError("register-window, marching and stage kernels need 16-byte aligned states and strides")
         rows, cols = self.module.gen.box(tile)
         self.params.tb_max = codegen.tile_steps(tile)
         if codegen.is_march(tile):
@@ -860,6 +866,20 @@ class StencilPlan:
             self.params.tile_z = max(1, codegen.tile_planes(tile))
             self.params.jobs_per_cta = 1
         self.params.box_planes = self.module.gen.box_depth(tile)
+        if stage:
+            # stage inputs and slope sums, from the stream's allocator for the
+            # time of the launches
+            keep = self.new_state(3) if self.integrator > 1 else None
+            buf = [None] * 3 if keep is None else [keep[k].data_ptr() for k in range(3)]
+            _native.check(
+                _native.lib().prml_fdm_run_stages(
+                    self._step_kernel(tile), tile[2], tile[4], ctypes.byref(self.params), self.integrator, y0,
+                    y0_bstride, traj, traj_bstride, traj_step_stride, wa, wb, self.inst, buf[0], buf[1], buf[2],
+                    n_steps, save_every, float(t0), float(dt), self.stream_handle(),
+                ),
+                "fdm run (stages)",
+            )
+            return
         _native.check(
             _native.lib().prml_fdm_run(
                 self._step_kernel(tile), tile[2], tile[0], tile[1], rows, cols, self.module.gen.box_planes(tile),
@@ -957,6 +977,9 @@ class StencilPlan:
 
         sms = _torch.cuda.get_device_properties(self.device).multi_processor_count
         cands = list(self.module.gen.step_kernels) + list(getattr(self.module.gen, "march_kernels", {}))
+        stage = list(getattr(self.module.gen, "stage_kernels", {}))
+        if stage and 3 * self.batch * self.inst * self.esize <= STAGE_WORK_BYTES:
+            cands += stage
         reps = 16  # a multiple of every temporal block; best of 3 rounds per tile
         # timing launches read boundary table 0 only: a time-dependent run's
         # tables may cover fewer half steps than the timing launches take
@@ -977,7 +1000,7 @@ class StencilPlan:
                 # fewer CTAs per SM that each walk several tiles and stage the
                 # next tile while computing the current one
                 # (marching jobs are sized by their rows instead)
-                caps = [0] + [sms * c for c in (2, 4, 8) if c < occ.value and not codegen.is_march(tile)]
+                caps = [0] + [sms * c for c in (2, 4, 8) if c < occ.value and not (codegen.is_march(tile) or codegen.is_stage(tile))]
 
                 def go(n, tile=tile):
                     self._launch(

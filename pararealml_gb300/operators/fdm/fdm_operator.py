@@ -22,7 +22,8 @@ GB300-side keyword-only options:
   solve (``numerical_integrator.py:135-270``) over right-hand-side kernel
   evaluations, with scipy.optimize.newton's warnings and error.
 * ``op_order``: ``"fused"`` (default) or ``"reference"``.  Fused order
-  evaluates the Cartesian Laplacian as one neighbour sum, uses explicit
+  evaluates the Cartesian Laplacian as one neighbour sum (on 3D meshes as
+  the sum of the second differences, scaled once), uses explicit
   multiply-adds and combines the integrator's stages from unscaled slopes
   (a stage-invariant RK4 step is y + dt f): about half the floating-point
   operations of the reference's numpy order, each result within a few
