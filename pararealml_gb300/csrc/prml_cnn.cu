@@ -284,6 +284,30 @@ __global__ void __launch_bounds__(256) reduce_parts(const float* __restrict__ pa
   }
 }
 
+/* Sums the partials of mid_wgrad_tc (dW [9][co][ci], then the 32 bias sums per
+ * part) as reduce_parts does, and stores dW as [9][ci][co] and db: one launch
+ * where reducing, transposing and the bias gradient took four. */
+__global__ void __launch_bounds__(256) reduce_wgrad(const float* __restrict__ partial, int parts,
+                                                    float* __restrict__ dw, float* __restrict__ db) {
+  constexpr int n = 9 * HC * HC + HC;
+  __shared__ float red[8][32];
+  const int i = blockIdx.x * 32 + threadIdx.x; /* n is a multiple of 32 */
+  float s = 0.f;
+  for (int k = threadIdx.y; k < parts; k += 8) s += partial[(long long)k * n + i];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0) return;
+  float t = 0.f;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) t += red[r][threadIdx.x];
+  if (i >= 9 * HC * HC) {
+    db[i - 9 * HC * HC] = t;
+  } else {
+    const int tap = i / (HC * HC), co = (i / HC) % HC, ci = i % HC;
+    dw[tap * HC * HC + ci * HC + co] = t;
+  }
+}
+
 /* [9][co][ci] -> [9][ci][co] (the wgrad GEMM's output is co-major) */
 __global__ void wgrad_transpose(const float* __restrict__ in, float* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -806,7 +830,7 @@ int prml_cnn_mid_dgrad(const void* g, const void* wd, const void* mask, void* gx
   return last("prml_cnn_mid_dgrad");
 }
 
-long long prml_cnn_wgrad_scratch_elems(int parts) { return (long long)parts * 9 * HC * HC + 9 * HC * HC; }
+long long prml_cnn_wgrad_scratch_elems(int parts) { return (long long)parts * (9 * HC * HC + HC) + 9 * HC * HC; }
 
 int prml_cnn_mid_wgrad(const void* x, const void* g, float* dw, float* db, int parts, float* scratch,
                        int B, int H, int W, void* stream) {
@@ -817,14 +841,15 @@ int prml_cnn_mid_wgrad(const void* x, const void* g, float* dw, float* db, int p
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int n = 9 * HC * HC;
   float* co_major = scratch + (long long)parts * n;
-  int used = parts;
   if (prml_cnn_tc_enabled()) {
+    int used = parts;
     rc = prml_cnn_mid_wgrad_tc(x, g, scratch, parts, &used, B, H, W, stream);
     if (rc) return rc;
-  } else {
-    mid_wgrad<<<parts, 288, WG_SMEM, s>>>(static_cast<const bf16*>(x), static_cast<const bf16*>(g), scratch, B, H, W);
+    reduce_wgrad<<<9 * HC + 1, dim3(32, 8), 0, s>>>(scratch, used, dw, db);
+    return last("prml_cnn_mid_wgrad");
   }
-  reduce_parts<<<(n + 31) / 32, dim3(32, 8), 0, s>>>(scratch, used, n, co_major, 1.f);
+  mid_wgrad<<<parts, 288, WG_SMEM, s>>>(static_cast<const bf16*>(x), static_cast<const bf16*>(g), scratch, B, H, W);
+  reduce_parts<<<(n + 31) / 32, dim3(32, 8), 0, s>>>(scratch, parts, n, co_major, 1.f);
   wgrad_transpose<<<(n + 255) / 256, 256, 0, s>>>(co_major, dw);
   channel_sum<<<parts, 256, 0, s>>>(static_cast<const bf16*>(g), (long long)B * H * W, scratch);
   reduce_parts<<<1, dim3(32, 8), 0, s>>>(scratch, parts, HC, db, 1.f);

@@ -2,23 +2,44 @@
  * 32 -> 32 channel 3x3 convolutions of the residual CNN on the 5th-generation
  * tensor cores (tcgen05, accumulators in tensor memory).
  *
- * Implicit GEMM per tile: M = 128 pixels (one row segment of one image),
- * N = 32 output channels, K = 9 taps x 32 input channels, issued as
- * 18 tcgen05.mma.kind::f16 (bf16 x bf16 -> f32, M128 N32 K16).
+ * Implicit GEMM: M = 128 pixels (one row segment of one image), K = 32 input
+ * channels of one column tap.  One staged input row feeds the (up to) three
+ * output rows around it at once: N = 3 x 32 output channels, the weights of
+ * the three row taps side by side, accumulated into three neighbouring
+ * 32-column accumulators in tensor memory.  So an input row costs 6
+ * tcgen05.mma.kind::f16 (bf16 x bf16 -> f32, M128 N96 K16; 3 column taps x 2
+ * halves of K).  What bounds a narrow MMA is reading A (128 pixels) from
+ * shared memory, not N: 18 MMAs of N = 32 per output row took 1200 cycles a
+ * tile and were the bound.  Each output still sums its 9 taps x 2 halves in
+ * the same order, from an accumulator that the epilogue left zeroed.  Only
+ * MMAs of one shape and accumulator are pipelined in order, so the next input
+ * row, whose accumulators lie one row further, waits for this one's MMAs (the
+ * commit that frees the row); the other CTA of the SM fills the gap.
+ * Measured, a layer of 16 images of 257^2: forward 56 -> 35 us, data gradient
+ * 58 -> 39 (135 MB read and written: 20 us), the CTA's chain of row loads,
+ * MMAs and epilogue being what is left (35 with the MMAs taken out before); of
+ * one image 21 -> 10.
  *
- * Work item: a band of up to 16 output rows of one 128-pixel column segment.
- * A CTA walks down the band; the input rows stream through a ring of 8
- * staged rows, so each output row costs one new input row: ONE TMA box load
- * of 130 whole pixels (64 bytes each, zero filled outside the image) with
- * the 64-byte swizzle.  That is the SWIZZLE_64B K-major canonical layout
- * (rows of 64 bytes = all 32 input channels, 8-row groups 512 bytes apart),
- * so the A matrix of tap (dy, dx) and K half kk starts at pixel dx, byte
- * 32 kk of the row for dy.  B operand: the packed weights [tap][n][k],
- * staged once per CTA as [tap][chunk][n][8] (no swizzle).
+ * Work item: a band of output rows of one 128-pixel column segment (band_rows
+ * chooses the band).  A CTA walks down the band; the input rows stream through
+ * a ring of 8 staged rows: ONE TMA box load of 130 whole pixels (64 bytes
+ * each, zero filled outside the image) with the 64-byte swizzle.  That is the
+ * SWIZZLE_64B K-major canonical layout (rows of 64 bytes = all 32 input
+ * channels, 8-row groups 512 bytes apart), so the A matrix of column tap dx
+ * and K half kk starts at pixel dx, byte 32 kk.  B operand: the packed weights
+ * [dx][chunk][row tap, n][8], staged once per CTA (no swizzle).
+ *
+ * Up to TAIL_W columns left over by the 128-pixel segments (rows of 2^k + 1
+ * vertices leave one) are not a segment of their own, which would spend a
+ * whole tile per row on them: a tail item is 16 rows x 8 pixels as one M =
+ * 128 tile.  Its box of 18 rows x 16 pixels is staged at 1024 bytes a row, so
+ * the 8-row groups of the A matrix are 1024 bytes apart and row tap dy is a
+ * start one staged row further.  257-wide rows: 3 tiles a row before, 2 1/16
+ * now.
  *
  * Roles per CTA (320 threads): warp 8 issues the row loads, warp 9 issues
- * the MMAs into one of four 32-column TMEM accumulators and releases each
- * row (tcgen05.commit) once the last tile that reads it has been issued, and
+ * the MMAs into one of eight 32-column TMEM accumulators and releases each
+ * row (tcgen05.commit) once its MMAs have been issued, and
  * two epilogue warpgroups (warps 0-3 and 4-7, alternating tiles; warp w reads
  * TMEM lanes 32 (w mod 4) ..) read an accumulator back with tcgen05.ld, apply
  * bias + ReLU (forward) or the ReLU mask of the layer input (data gradient)
@@ -44,28 +65,35 @@ constexpr unsigned TX_BYTES = SEG * PIX_BYTES; /* one staged row: 8320 bytes */
 /* rows start on 1024-byte boundaries (the swizzle pattern repeats every 512) */
 constexpr int ROW_BYTES = (int)((TX_BYTES + 1023) / 1024 * 1024);
 constexpr int NROW = 8;                    /* staged-row ring (a power of two) */
-constexpr int BAND = 16;                   /* output rows per work item */
-constexpr int W_BYTES = 9 * 4 * HC * 16;   /* [tap][chunk][n][8] */
-constexpr int NACC = 4;
-constexpr int TMEM_COLS = 128;             /* NACC x 32 columns */
+constexpr int BAND = 16;                   /* most output rows per work item; rows of a tail item */
+constexpr int TAIL_W = 8;                  /* most columns of a tail item */
+constexpr int TAIL_SEG = 16;               /* staged pixels per row of a tail item (TAIL_W + 2 used) */
+constexpr int TAIL_PITCH = TAIL_SEG * PIX_BYTES;
+constexpr unsigned TAIL_TX = (BAND + 2) * TAIL_PITCH;
+constexpr int W_BYTES = 9 * 4 * HC * 16;   /* [dx][chunk][dy' n][8], dy' = 2 - dy */
+constexpr int W_CHUNK = 3 * HC * 16;       /* bytes of one chunk (8 input channels) of one column tap */
+constexpr int NACC = 8;
+constexpr int TMEM_COLS = 256;             /* NACC x 32 columns: two CTAs hold an SM's tensor memory */
 constexpr int EPI_GROUPS = 2;              /* epilogue warpgroups, alternating tiles */
 constexpr int TMA_WARP = 4 * EPI_GROUPS, MMA_WARP = TMA_WARP + 1;
 constexpr int THREADS = (MMA_WARP + 1) * 32;
 static_assert(NACC % EPI_GROUPS == 0, "each group owns whole accumulators");
-constexpr int BAR_BYTES = 256;
+constexpr int BAR_BYTES = 384;
 constexpr int SMEM_BYTES = NROW * ROW_BYTES + W_BYTES + BAR_BYTES + HC * 4 + 16 + 1024; /* + alignment slack */
 constexpr unsigned long long kWaitNs = 2000000000ull; /* 2 s */
 static_assert(ROW_BYTES % 1024 == 0, "swizzled TMA destinations start on 1024-byte boundaries");
 static_assert((NROW * ROW_BYTES + W_BYTES) % 128 == 0, "weights and barriers aligned");
-static_assert((2 * NROW + 2 * NACC) * 8 <= BAR_BYTES, "barrier area");
+static_assert((2 * NROW + 2 * NACC + 1) * 8 <= BAR_BYTES, "barrier area");
+static_assert(TAIL_TX <= 2 * ROW_BYTES && TAIL_PITCH == 1024, "a tail box fills two ring slots, rows on 1024 bytes");
 static_assert(NROW >= 4 && (NROW & (NROW - 1)) == 0, "ring of a power of two >= 4 rows");
 static_assert((HC * 16 >> 4) < (1 << 14) && (512 >> 4) < (1 << 14), "descriptor offsets fit 14 bits");
 static_assert(NROW * ROW_BYTES + W_BYTES < (1 << 18), "descriptor start fields (addr >> 4, 14 bits) never carry");
 
 /* instruction descriptor, kind::f16: D f32, A bf16, B bf16, both K-major,
- * N = 32, M = 128 */
-constexpr unsigned kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(HC >> 3) << 17) |
-                            ((unsigned)(TM >> 4) << 24);
+ * M = 128, N = 32 blocks */
+__device__ __forceinline__ constexpr unsigned idesc(int blocks) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(blocks * (HC >> 3)) << 17) | ((unsigned)(TM >> 4) << 24);
+}
 
 __device__ int g_cnn_tc_status;
 
@@ -130,17 +158,17 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned 
  * writes it, so a start shifted by whole pixels or by 32 bytes inside a row
  * needs no base offset (measured: base offset 0 matches the reference
  * convolution, the address-derived one does not). */
-__device__ __forceinline__ unsigned long long smem_desc_sw64(unsigned addr) {
-  return (unsigned long long)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((unsigned long long)(512u >> 4) << 32) |
+__device__ __forceinline__ unsigned long long smem_desc_sw64(unsigned addr, unsigned sbo = 512u) {
+  return (unsigned long long)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((unsigned long long)(sbo >> 4) << 32) |
          (1ull << 46) | (4ull << 61);
 }
 
-__device__ __forceinline__ void mma_f16(unsigned d_tmem, unsigned long long a, unsigned long long b,
+__device__ __forceinline__ void mma_f16(unsigned d_tmem, unsigned long long a, unsigned long long b, unsigned id,
                                         unsigned accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate)
+      "l"(a), "l"(b), "r"(id), "r"(accumulate)
       : "memory");
 }
 
@@ -165,23 +193,76 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+/* zeroes 32 columns of the warp's 32 lanes */
+__device__ __forceinline__ void tmem_zero32(unsigned taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
+      "r"(0)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-struct Item {
-  int b, r0, rows, x0;
+/* Work items of a layer: bands of `band` rows of the 128-pixel segments, then
+ * the tail items. */
+struct Items {
+  int segs, nbands, band, main, groups, total, H, W;
 };
 
-/* work item t: image b, band of output rows [r0, r0 + rows), segment x0 */
-__device__ __forceinline__ Item item_at(int t, int segs, int nbands, int H) {
-  const int per_img = segs * nbands;
+struct Item {
+  int b, r0, rows, x0; /* image, output rows [r0, r0 + rows), first column */
+  bool tail;           /* a tail item: rows x (at most TAIL_W) columns, one tile */
+  __device__ __forceinline__ int tiles() const { return tail ? 1 : rows; }
+};
+
+__host__ __device__ __forceinline__ Items make_items(int B, int H, int W, int band) {
+  Items n;
+  const int left = W % TM;
+  const bool tail = left >= 1 && left <= TAIL_W;
+  n.segs = W / TM + (left && !tail ? 1 : 0);
+  n.band = band;
+  n.nbands = (H + band - 1) / band;
+  n.groups = tail ? (H + BAND - 1) / BAND : 0;
+  n.main = B * n.segs * n.nbands;
+  n.total = n.main + B * n.groups;
+  n.H = H;
+  n.W = W;
+  return n;
+}
+
+/* Rows of a band: the rows a slot takes when all rows of all segments are
+ * dealt evenly in as few rounds of at most BAND rows as it takes.  Fixed 16-row
+ * bands left a batch of one 257^2 image 51 of the 304 slots busy for 16 rows
+ * each (21 us a layer) and 16 images 1.8 rounds. */
+int band_rows(int B, int H, int W, int slots) {
+  const Items one = make_items(B, H, W, BAND);
+  const long long total = (long long)B * H * (one.segs > 0 ? one.segs : 1);
+  const long long rounds = (total + (long long)slots * BAND - 1) / ((long long)slots * BAND);
+  const long long band = (total + slots * rounds - 1) / (slots * rounds);
+  return (int)(band < 1 ? 1 : (band > BAND ? BAND : band));
+}
+
+__device__ __forceinline__ Item item_at(int t, const Items& n) {
   Item it;
+  it.tail = t >= n.main;
+  if (it.tail) {
+    t -= n.main;
+    it.b = t / n.groups;
+    it.r0 = (t - it.b * n.groups) * BAND;
+    it.x0 = n.segs * TM;
+    it.rows = n.H - it.r0 < BAND ? n.H - it.r0 : BAND;
+    return it;
+  }
+  const int per_img = n.segs * n.nbands;
   it.b = t / per_img;
   const int r = t - it.b * per_img;
-  const int band = r / segs;
-  it.x0 = (r - band * segs) * TM;
-  it.r0 = band * BAND;
-  it.rows = H - it.r0 < BAND ? H - it.r0 : BAND;
+  const int band = r / n.segs;
+  it.x0 = (r - band * n.segs) * TM;
+  it.r0 = band * n.band;
+  it.rows = n.H - it.r0 < n.band ? n.H - it.r0 : n.band;
   return it;
 }
 
@@ -189,10 +270,11 @@ __device__ __forceinline__ Item item_at(int t, int segs, int nbands, int H) {
  * w: [tap][n][k] bf16 (n = output channel). */
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant__ CUtensorMap xmap,
+                                                          const __grid_constant__ CUtensorMap tmap,
                                                           const bf16* __restrict__ w,
                                                           const float* __restrict__ bias,
                                                           const bf16* __restrict__ mask, bf16* __restrict__ y,
-                                                          int B, int H, int W) {
+                                                          const Items n) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
   unsigned char* rows = base;
@@ -202,23 +284,20 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
   unsigned long long* empty = bars + NROW;         /* [NROW] */
   unsigned long long* accfull = bars + 2 * NROW;   /* [NACC] */
   unsigned long long* accempty = accfull + NACC;   /* [NACC] */
+  unsigned long long* done = accempty + NACC;      /* all MMAs complete */
   float* bias_s = reinterpret_cast<float*>(wsm + W_BYTES + BAR_BYTES);
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bias_s + HC);
   __shared__ int abort_flag;
   __shared__ int loads_issued;  /* row loads issued by the producer */
   __shared__ int loads_waited;  /* row loads the MMA warp has seen land */
-  __shared__ int tiles_issued;  /* tiles whose MMAs were issued */
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int segs = (W + TM - 1) / TM;
-  const int nbands = (H + BAND - 1) / BAND;
-  const int items = B * segs * nbands;
 
-  /* weights [tap][n][k] -> [tap][chunk][n][8], bias */
+  /* weights [dy][dx][n][k] -> [dx][chunk][2 - dy][n][8], bias */
   for (int i = tid; i < 9 * HC * 4; i += THREADS) {
-    const int tap = i / (HC * 4), rem = i - tap * HC * 4, n = rem >> 2, c = rem & 3;
-    const uint4 v = *reinterpret_cast<const uint4*>(w + (tap * HC + n) * HC + c * 8);
-    *reinterpret_cast<uint4*>(wsm + ((tap * 4 + c) * HC + n) * 16) = v;
+    const int tap = i / (HC * 4), rem = i - tap * HC * 4, co = rem >> 2, c = rem & 3;
+    const uint4 v = *reinterpret_cast<const uint4*>(w + (tap * HC + co) * HC + c * 8);
+    *reinterpret_cast<uint4*>(wsm + (((tap % 3) * 4 + c) * 3 * HC + (2 - tap / 3) * HC + co) * 16) = v;
   }
   if (MODE == 0 && tid < HC) bias_s[tid] = bias[tid];
   if (tid == 0) {
@@ -230,10 +309,10 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
       bar_init(&accfull[a], 1);
       bar_init(&accempty[a], 4 * 32);
     }
+    bar_init(done, 1);
     abort_flag = 0;
     loads_issued = 0;
     loads_waited = 0;
-    tiles_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   /* generic-proxy weight stores must be visible to the tensor cores */
@@ -248,80 +327,116 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = *tmem_slot;
+  if (warp < 4)
+    for (int a = 0; a < NACC; ++a) tmem_zero32(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(a * HC));
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 
   if (warp == TMA_WARP) {
-    /* ---- row loads */
+    /* ---- row loads; a tail box takes two ring slots, the first one even
+     * (the slot skipped for that completes without a copy) */
     if (lane == 0) {
       int L = 0;
-      for (int t = blockIdx.x; t < items && !abort_flag; t += gridDim.x) {
-        const Item it = item_at(t, segs, nbands, H);
-        for (int j = 0; j < it.rows + 2; ++j, ++L) {
+      bool ok = true;
+      for (int t = blockIdx.x; t < n.total && ok; t += gridDim.x) {
+        const Item it = item_at(t, n);
+        const int loads = it.tail ? 2 + (L & 1) : it.rows + 2;
+        for (int j = 0; j < loads; ++j, ++L) {
           const int q = L % NROW;
           unsigned char* dst = rows + q * ROW_BYTES;
-          if (!bar_wait(&empty[q], ((L / NROW) & 1) ^ 1) || *(volatile int*)&abort_flag ||
-              (saddr(dst) & 1023u)) { /* the last test: never issue a misaligned copy */
-            atomicExch(&abort_flag, 1);
-            break;
+          ok = bar_wait(&empty[q], ((L / NROW) & 1) ^ 1) && !*(volatile int*)&abort_flag &&
+               (saddr(dst) & 1023u) == 0; /* the last test: never issue a misaligned copy */
+          if (ok && it.tail && loads - j == 2) /* the box also writes the next slot */
+            ok = bar_wait(&empty[q + 1], (((L + 1) / NROW) & 1) ^ 1);
+          if (!ok) break;
+          if (!it.tail) {
+            bar_expect_tx(&full[q], TX_BYTES);
+            tma_row(dst, &xmap, it.x0 - 1, it.r0 - 1 + j, it.b, &full[q]);
+          } else if (loads - j == 2) {
+            bar_expect_tx(&full[q], TAIL_TX);
+            tma_row(dst, &tmap, it.x0 - 1, it.r0 - 1, it.b, &full[q]);
+          } else {
+            bar_arrive(&full[q]);
           }
-          bar_expect_tx(&full[q], TX_BYTES);
-          tma_row(dst, &xmap, it.x0 - 1, it.r0 - 1 + j, it.b, &full[q]);
           loads_issued = L + 1;
         }
       }
+      if (!ok) atomicExch(&abort_flag, 1);
     }
   } else if (warp == MMA_WARP) {
     /* ---- MMA issuer */
     if (lane == 0) {
       const unsigned wbase = saddr(wsm);
-      int L0 = 0, T = 0;
+      int L = 0, T = 0; /* ring slots and accumulators used so far */
       bool ok = (wbase & 15u) == 0;
-      /* ring rows are ROW_BYTES apart: slot q's descriptor is adesc0 + q * (ROW_BYTES >> 4) */
+      /* descriptors are linear in the start address (field = addr >> 4, no
+       * carry for shared addresses): ring slots are ROW_BYTES apart */
       const unsigned long long adesc0 = smem_desc_sw64(saddr(rows));
-      const unsigned long long bdesc = smem_desc(wbase, HC * 16, 128);
-      auto adesc = [&](int L) {
-        return adesc0 + (unsigned long long)((L & (NROW - 1)) * (ROW_BYTES >> 4));
-      };
-      auto landed = [&](int L) {
-        if (!bar_wait(&full[L % NROW], (L / NROW) & 1)) return false;
-        loads_waited = L + 1;
+      const unsigned long long tdesc0 = smem_desc_sw64(saddr(rows), TAIL_PITCH);
+      const unsigned long long bdesc = smem_desc(wbase, W_CHUNK, 128);
+      auto landed = [&](int l) {
+        if (!bar_wait(&full[l % NROW], (l / NROW) & 1)) return false;
+        loads_waited = l + 1;
         return true;
       };
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        const Item it = item_at(t, segs, nbands, H);
-        ok = landed(L0) && landed(L0 + 1);
-        for (int i = 0; i < it.rows && ok; ++i, ++T) {
-          const int a = T % NACC;
-          ok = landed(L0 + i + 2) && bar_wait(&accempty[a], ((T / NACC) & 1) ^ 1) &&
-               !*(volatile int*)&abort_flag;
+      auto acc_free = [&](int a) {
+        return bar_wait(&accempty[a % NACC], ((a / NACC) & 1) ^ 1) && !*(volatile int*)&abort_flag;
+      };
+      /* column tap dx, K half kk of one A row for row-tap blocks [blk, blk + cnt) into the accumulator of tile a */
+      auto mma = [&](unsigned long long ar, int dx, int kk, int a, int blk, int cnt) {
+        mma_f16(tmem + (unsigned)((a % NACC) * HC), ar + (unsigned long long)((dx * PIX_BYTES + kk * 32) >> 4),
+                bdesc + (unsigned long long)(((dx * 4 + 2 * kk) * W_CHUNK + blk * HC * 16) >> 4), idesc(cnt), 1u);
+      };
+      for (int t = blockIdx.x; t < n.total && ok; t += gridDim.x) {
+        const Item it = item_at(t, n);
+        if (it.tail) {
+          if (L & 1) {
+            if (!(ok = landed(L))) break;
+            bar_arrive(&empty[L % NROW]);
+            ++L;
+          }
+          ok = landed(L) && landed(L + 1) && acc_free(T);
           if (!ok) break;
           tc_fence_after();
-          const unsigned d = tmem + (unsigned)(a * HC);
-          /* descriptors are linear in the start address (field = addr >> 4,
-           * no carry for shared addresses), so each MMA's operands are a
-           * constant add to the base descriptor of its row slot / weights */
-          const unsigned long long r0 = adesc(L0 + i);
-          const unsigned long long r1 = adesc(L0 + i + 1);
-          const unsigned long long r2 = adesc(L0 + i + 2);
+          const unsigned long long ar = tdesc0 + (unsigned long long)((L % NROW) * (ROW_BYTES >> 4));
 #pragma unroll
-          for (int tap = 0; tap < 9; ++tap) {
-            const unsigned long long ra = tap < 3 ? r0 : (tap < 6 ? r1 : r2);
+          for (int tap = 0; tap < 9; ++tap)
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk)
-              mma_f16(d, ra + (unsigned long long)(((tap % 3) * PIX_BYTES + kk * 32) >> 4),
-                      bdesc + (unsigned long long)(((tap * 4 + 2 * kk) * HC * 16) >> 4),
-                      (tap > 0 || kk > 0) ? 1u : 0u);
-          }
-          mma_commit(&accfull[a]);                /* the accumulator is ready */
-          mma_commit(&empty[(L0 + i) % NROW]);    /* row y-1 is read for the last time */
-          tiles_issued = T + 1;
+              mma(ar + (unsigned long long)((tap / 3) * (TAIL_PITCH >> 4)), tap % 3, kk, T, 2 - tap / 3, 1);
+          mma_commit(&accfull[T % NACC]);
+          mma_commit(&empty[L % NROW]);
+          mma_commit(&empty[(L + 1) % NROW]);
+          L += 2;
+          ++T;
+          continue;
         }
-        if (!ok) break;
-        /* the band's last two rows are free once its last MMAs are done */
-        mma_commit(&empty[(L0 + it.rows) % NROW]);
-        mma_commit(&empty[(L0 + it.rows + 1) % NROW]);
-        L0 += it.rows + 2;
+        for (int j = 0; j < it.rows + 2 && ok; ++j, ++L) {
+          /* input row j feeds output rows lo .. hi of the band: row i through
+           * row tap j - i, weight block 2 - (j - i) */
+          const int lo = j > 2 ? j - 2 : 0, hi = j < it.rows ? j : it.rows - 1;
+          ok = landed(L) && (j >= it.rows || acc_free(T + j)) &&
+               (j == 0 || bar_wait(&empty[(L - 1) % NROW], ((L - 1) / NROW) & 1));
+          if (!ok) break;
+          tc_fence_after();
+          const unsigned long long ar = adesc0 + (unsigned long long)((L % NROW) * (ROW_BYTES >> 4));
+          /* their accumulators may wrap around the ring */
+          const int blk = 2 - (j - lo), cnt = hi - lo + 1, room = NACC - (T + lo) % NACC;
+          const int c0 = cnt < room ? cnt : room;
+#pragma unroll
+          for (int k = 0; k < 6; ++k) {
+            mma(ar, k >> 1, k & 1, T + lo, blk, c0);
+            if (c0 < cnt) mma(ar, k >> 1, k & 1, T + lo + c0, blk + c0, cnt - c0);
+          }
+          if (j >= 2) mma_commit(&accfull[(T + j - 2) % NACC]); /* that output row is complete */
+          mma_commit(&empty[L % NROW]);
+        }
+        T += it.rows;
       }
       if (!ok) atomicExch(&abort_flag, 1);
+      mma_commit(done); /* arrives once every MMA issued above has completed */
+      bar_wait(done, 0);
     }
   } else {
     /* ---- epilogue: group g takes the tiles T with T mod EPI_GROUPS == g;
@@ -329,9 +444,10 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
     const int group = warp >> 2, wq = warp & 3;
     int T = 0;
     bool go = true;
-    for (int t = blockIdx.x; t < items && go; t += gridDim.x) {
-      const Item it = item_at(t, segs, nbands, H);
-      for (int i = 0; i < it.rows; ++i, ++T) {
+    for (int t = blockIdx.x; t < n.total && go; t += gridDim.x) {
+      const Item it = item_at(t, n);
+      const int tiles = it.tiles();
+      for (int i = 0; i < tiles; ++i, ++T) {
         if (T % EPI_GROUPS != group) continue;
         const int a = T % NACC;
         const bool ok = bar_wait(&accfull[a], (T / NACC) & 1);
@@ -342,12 +458,15 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
         }
         tc_fence_after();
         float v[32];
-        tmem_ld32(tmem + ((unsigned)(wq * 32) << 16) + (unsigned)(a * HC), v);
+        const unsigned acc = tmem + ((unsigned)(wq * 32) << 16) + (unsigned)(a * HC);
+        tmem_ld32(acc, v);
+        tmem_zero32(acc); /* the next tile's first products add to zero */
         tc_fence_before();
         bar_arrive(&accempty[a]);
-        const int gx = it.x0 + wq * 32 + lane;
-        if (gx < W) {
-          const long long p = ((long long)it.b * H + it.r0 + i) * W + gx;
+        const int m = wq * 32 + lane;
+        const int gx = it.x0 + (it.tail ? m % TAIL_W : m), gy = it.tail ? m / TAIL_W : i;
+        if (gx < n.W && gy < it.rows) {
+          const long long p = ((long long)it.b * n.H + it.r0 + gy) * n.W + gx;
           if (MODE == 0) {
 #pragma unroll
             for (int k = 0; k < 32; ++k) v[k] = fmaxf(v[k] + bias_s[k], 0.f);
@@ -387,10 +506,6 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
       /* row loads issued but never seen by the MMA warp */
       for (int j = loads_waited; j < loads_issued; ++j) bar_wait(&full[j % NROW], (j / NROW) & 1);
     }
-    if (warp == MMA_WARP && lane == 0 && tiles_issued > 0) {
-      const int j = tiles_issued - 1;
-      bar_wait(&accfull[j % NACC], (j / NACC) & 1);
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -399,69 +514,65 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
-/* ---- weight gradient of the 32 -> 32 convolutions ---------------------------
+/* ---- weight and bias gradient of the 32 -> 32 convolutions ------------------
  * dW[dy][dx][co][ci] = sum over pixels p of g[p][co] x[p + (dy - 1, dx - 1)][ci]
  * (x zero outside the image) as tcgen05 MMAs whose K is pixels.  D (M = 128,
- * N = 32, f32 in TMEM) row 32 j + ci holds the column shift j - 1 of input
- * channel ci for every output channel; j = 3 (a shift of +2) is computed and
- * discarded, so one MMA covers a kernel row's three taps.  One accumulator
- * per kernel row dy (96 TMEM columns).  Both operands are the staged NHWC
- * rows read MN-major with the 64-byte swizzle (a pixel's 32 channels are one
- * 64-byte row of a swizzle atom, 8 pixels one 512-byte atom): A = the input
- * row y + dy - 1 from one pixel left of the K block, its four 32-row MN
- * blocks one pixel (64 bytes, the leading byte offset) apart, 8-pixel K
- * groups 512 bytes (the stride byte offset) apart; B = the gradient row y.
- * A CTA walks (image, band, 128-pixel segment) items as the convolution does,
- * accumulates over all of them, and writes its partial dW [tap][co][ci]
- * once at the end.  Roles: warp 4 loads rows (input rows through the ring of
- * NROW, gradient rows through a ring of WG_NG), warp 5 issues the MMAs,
- * warps 0-3 read the accumulators back.  Waits are bounded as in the
- * convolution. */
+ * f32 in TMEM) row 32 j + ci holds the column shift j - 1 of input channel ci;
+ * j = 3 (a shift of +2) is computed and discarded, so one MMA covers a kernel
+ * row's three taps.  One staged input row meets the (up to) three gradient
+ * rows around it at once: N = 3 x 32 output channels, one 32-column
+ * accumulator per kernel row (dy in columns 32 (2 - dy) ..), so an input row
+ * costs 8 MMAs of N = 96 where an output row took 24 of N = 32.  Both operands
+ * are the staged NHWC rows read MN-major with the 64-byte swizzle (a pixel's
+ * 32 channels are one 64-byte row of a swizzle atom, 8 pixels one 512-byte
+ * atom): A = the input row from one pixel left of the K block, its four 32-row
+ * MN blocks one pixel (64 bytes, the leading byte offset) apart, 8-pixel K
+ * groups 512 bytes (the stride byte offset) apart; B = gradient rows, MN
+ * blocks one ring slot apart.  A tail item (16 rows x 8 pixels) is one K of
+ * 128 pixels: its 8-pixel groups are rows, 1024 bytes apart in A.
+ * A CTA walks items as the convolution does, accumulates over all of them, and
+ * writes its partial dW [tap][co][ci] and bias sums once at the end.  Roles:
+ * warp 4 loads rows (input rows through a ring of WG_NX, gradient rows through
+ * a ring of WG_NG), warp 5 issues the MMAs, warps 0-3 sum the staged gradient
+ * rows per channel (a pass of its own over the gradient took 20 us of a
+ * layer's 90 at 16 x 257^2) and read the accumulators back.  Waits are bounded
+ * as in the convolution.
+ * Measured, 16 images of 257^2: 56 -> 35 us, and 36 us of four more launches
+ * (bias pass, two reductions, transposition) became 7 (reduce_wgrad). */
 constexpr int WG_G_BYTES = TM * PIX_BYTES; /* one gradient row, 8192 bytes */
-constexpr int WG_NG = 4;
+constexpr int WG_NX = 4, WG_NG = 8;
+constexpr int WG_PART = 9 * HC * HC + HC;  /* floats of a CTA's partial: dW, then the bias sums */
 constexpr int WG_TMEM_COLS = 128;          /* 3 x 32 used */
 constexpr int WG_TMA_WARP = 4, WG_MMA_WARP = 5;
 constexpr int WG_THREADS = 6 * 32;
 /* + alignment slack + room for reads of the discarded shift past a row */
-constexpr int WG_SMEM = NROW * ROW_BYTES + WG_NG * WG_G_BYTES + BAR_BYTES + 1024 + 2048;
-constexpr unsigned kIdescWg = kIdesc | (1u << 15) | (1u << 16); /* A and B MN-major */
+constexpr int WG_SMEM = WG_NX * ROW_BYTES + WG_NG * WG_G_BYTES + BAR_BYTES + 1024 + 2048;
+constexpr unsigned kMnMajor = (1u << 15) | (1u << 16); /* A and B MN-major */
 static_assert(WG_G_BYTES % 1024 == 0, "gradient rows start on 1024-byte boundaries");
-static_assert((2 * NROW + 2 * WG_NG + 1) * 8 <= BAR_BYTES, "barrier area");
-static_assert(NROW * ROW_BYTES + WG_NG * WG_G_BYTES + BAR_BYTES < (1 << 18), "descriptor start fields never carry");
+static_assert((2 * WG_NX + 2 * WG_NG + 1) * 8 <= BAR_BYTES, "barrier area");
+static_assert(BAND * TAIL_W * PIX_BYTES == WG_G_BYTES, "a tail item's gradient fills one slot");
+static_assert(WG_NX * ROW_BYTES + WG_NG * WG_G_BYTES + BAR_BYTES < (1 << 18), "descriptor start fields never carry");
 
 /* SWIZZLE_64B MN-major descriptor: MN blocks of 32 elements `lbo` bytes
- * apart, 8-row K groups 512 bytes apart */
-__device__ __forceinline__ unsigned long long smem_desc_mn_sw64(unsigned addr, unsigned lbo) {
+ * apart, 8-row K groups `sbo` bytes apart */
+__device__ __forceinline__ unsigned long long smem_desc_mn_sw64(unsigned addr, unsigned lbo, unsigned sbo = 512u) {
   return (unsigned long long)((addr >> 4) & 0x3FFFu) | ((unsigned long long)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((unsigned long long)(512u >> 4) << 32) | (1ull << 46) | (4ull << 61);
-}
-
-__device__ __forceinline__ void mma_f16_wg(unsigned d_tmem, unsigned long long a, unsigned long long b,
-                                           unsigned accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(kIdescWg), "r"(accumulate)
-      : "memory");
-}
-
-/* one gradient row: box {32, 128, 1, 1} at (0, x, y, b), 64-byte swizzle */
-__device__ __forceinline__ void tma_grow(void* dst, const CUtensorMap* map, int x, int y, int b,
-                                         unsigned long long* bar) {
-  tma_row(dst, map, x, y, b, bar);
+         ((unsigned long long)(sbo >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
 
 __global__ void __launch_bounds__(WG_THREADS, 2) mid_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
                                                               const __grid_constant__ CUtensorMap gmap,
-                                                              float* __restrict__ partial, int B, int H, int W) {
+                                                              const __grid_constant__ CUtensorMap xtail,
+                                                              const __grid_constant__ CUtensorMap gtail,
+                                                              float* __restrict__ partial, const Items n) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
   unsigned char* xrows = base;
-  unsigned char* grows = base + NROW * ROW_BYTES;
+  unsigned char* grows = base + WG_NX * ROW_BYTES;
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(grows + WG_NG * WG_G_BYTES);
-  unsigned long long* xfull = bars;                  /* [NROW] */
-  unsigned long long* xempty = bars + NROW;          /* [NROW] */
-  unsigned long long* gfull = bars + 2 * NROW;       /* [WG_NG] */
+  unsigned long long* xfull = bars;                  /* [WG_NX] */
+  unsigned long long* xempty = bars + WG_NX;         /* [WG_NX] */
+  unsigned long long* gfull = bars + 2 * WG_NX;      /* [WG_NG] */
   unsigned long long* gempty = gfull + WG_NG;        /* [WG_NG] */
   unsigned long long* done = gempty + WG_NG;         /* all MMAs complete */
   __shared__ unsigned tmem_slot;
@@ -469,18 +580,16 @@ __global__ void __launch_bounds__(WG_THREADS, 2) mid_wgrad_tc(const __grid_const
   __shared__ int xl_issued, xl_waited, gl_issued, gl_waited;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int segs = (W + TM - 1) / TM;
-  const int nbands = (H + BAND - 1) / BAND;
-  const int items = B * segs * nbands;
+  __shared__ float bias_sum[4][HC];
 
   if (tid == 0) {
-    for (int q = 0; q < NROW; ++q) {
+    for (int q = 0; q < WG_NX; ++q) {
       bar_init(&xfull[q], 1);
       bar_init(&xempty[q], 1);
     }
     for (int q = 0; q < WG_NG; ++q) {
       bar_init(&gfull[q], 1);
-      bar_init(&gempty[q], 1);
+      bar_init(&gempty[q], 1 + 4); /* the MMAs and the four summing warps */
     }
     bar_init(done, 1);
     abort_flag = 0;
@@ -497,34 +606,55 @@ __global__ void __launch_bounds__(WG_THREADS, 2) mid_wgrad_tc(const __grid_const
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = tmem_slot;
+  if (warp < 4)
+    for (int a = 0; a < 3; ++a) tmem_zero32(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(a * HC));
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 
   if (warp == WG_TMA_WARP) {
-    /* ---- row loads: input rows r0 - 1 .. r0 + rows, and after input row
-     * j the gradient row j - 2 (so an output row's inputs arrive together) */
+    /* ---- row loads: input rows r0 - 1 .. r0 + rows, after input row j the
+     * gradient row j (the last it meets); a tail item is one input box in two
+     * ring slots, the first one even, and one gradient box */
     if (lane == 0) {
       int L = 0, G = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        const Item it = item_at(t, segs, nbands, H);
-        for (int j = 0; j < it.rows + 2 && ok; ++j) {
-          const int q = L % NROW;
-          unsigned char* dst = xrows + q * ROW_BYTES;
-          ok = bar_wait(&xempty[q], ((L / NROW) & 1) ^ 1) && !*(volatile int*)&abort_flag &&
-               (saddr(dst) & 1023u) == 0;
-          if (!ok) break;
-          bar_expect_tx(&xfull[q], TX_BYTES);
-          tma_row(dst, &xmap, it.x0 - 1, it.r0 - 1 + j, it.b, &xfull[q]);
-          xl_issued = ++L;
-          if (j >= 2) {
-            const int qg = G % WG_NG;
-            unsigned char* gdst = grows + qg * WG_G_BYTES;
-            ok = bar_wait(&gempty[qg], ((G / WG_NG) & 1) ^ 1) && !*(volatile int*)&abort_flag &&
-                 (saddr(gdst) & 1023u) == 0;
-            if (!ok) break;
-            bar_expect_tx(&gfull[qg], WG_G_BYTES);
-            tma_grow(gdst, &gmap, it.x0, it.r0 + j - 2, it.b, &gfull[qg]);
-            gl_issued = ++G;
+      auto xslot = [&](int l) {
+        return bar_wait(&xempty[l % WG_NX], ((l / WG_NX) & 1) ^ 1) && !*(volatile int*)&abort_flag &&
+               (saddr(xrows + (l % WG_NX) * ROW_BYTES) & 1023u) == 0;
+      };
+      auto gload = [&](const CUtensorMap* map, int x, int y, int b) {
+        const int q = G % WG_NG;
+        unsigned char* dst = grows + q * WG_G_BYTES;
+        if (!bar_wait(&gempty[q], ((G / WG_NG) & 1) ^ 1) || *(volatile int*)&abort_flag || (saddr(dst) & 1023u))
+          return false;
+        bar_expect_tx(&gfull[q], WG_G_BYTES);
+        tma_row(dst, map, x, y, b, &gfull[q]);
+        gl_issued = ++G;
+        return true;
+      };
+      for (int t = blockIdx.x; t < n.total && ok; t += gridDim.x) {
+        const Item it = item_at(t, n);
+        if (it.tail) {
+          if (L & 1) {
+            if (!(ok = xslot(L))) break;
+            bar_arrive(&xfull[L % WG_NX]);
+            xl_issued = ++L;
           }
+          if (!(ok = xslot(L) && xslot(L + 1))) break;
+          bar_expect_tx(&xfull[L % WG_NX], TAIL_TX);
+          tma_row(xrows + (L % WG_NX) * ROW_BYTES, &xtail, it.x0 - 1, it.r0 - 1, it.b, &xfull[L % WG_NX]);
+          bar_arrive(&xfull[(L + 1) % WG_NX]);
+          xl_issued = L += 2;
+          ok = gload(&gtail, it.x0, it.r0, it.b);
+          continue;
+        }
+        for (int j = 0; j < it.rows + 2 && ok; ++j) {
+          if (!(ok = xslot(L))) break;
+          bar_expect_tx(&xfull[L % WG_NX], TX_BYTES);
+          tma_row(xrows + (L % WG_NX) * ROW_BYTES, &xmap, it.x0 - 1, it.r0 - 1 + j, it.b, &xfull[L % WG_NX]);
+          xl_issued = ++L;
+          if (j < it.rows) ok = gload(&gmap, it.x0, it.r0 + j, it.b);
         }
       }
       if (!ok) atomicExch(&abort_flag, 1);
@@ -532,64 +662,143 @@ __global__ void __launch_bounds__(WG_THREADS, 2) mid_wgrad_tc(const __grid_const
   } else if (warp == WG_MMA_WARP) {
     /* ---- MMA issuer */
     if (lane == 0) {
-      int L0 = 0, G0 = 0, T = 0;
+      int L = 0, G = 0;
       bool ok = true;
-      auto xlanded = [&](int L) {
-        if (!bar_wait(&xfull[L % NROW], (L / NROW) & 1)) return false;
-        xl_waited = L + 1;
+      auto xlanded = [&](int l) {
+        if (!bar_wait(&xfull[l % WG_NX], (l / WG_NX) & 1)) return false;
+        xl_waited = l + 1;
+        return !*(volatile int*)&abort_flag;
+      };
+      auto glanded = [&](int l) {
+        if (!bar_wait(&gfull[l % WG_NG], (l / WG_NG) & 1)) return false;
+        gl_waited = l + 1;
         return true;
       };
       const unsigned xbase = saddr(xrows), gbase = saddr(grows);
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        const Item it = item_at(t, segs, nbands, H);
-        /* K blocks holding pixels of the image: past it the gradient is
-         * zero (the last segment of a 257-wide row holds one pixel) */
-        const int ksteps = (W - it.x0 >= TM) ? TM / 16 : (W - it.x0 + 15) / 16;
-        ok = xlanded(L0) && xlanded(L0 + 1);
-        for (int i = 0; i < it.rows && ok; ++i, ++T) {
-          const int qg = (G0 + i) % WG_NG;
-          ok = xlanded(L0 + i + 2) && bar_wait(&gfull[qg], ((G0 + i) / WG_NG) & 1) &&
-               !*(volatile int*)&abort_flag;
-          if (!ok) break;
-          gl_waited = G0 + i + 1;
-          tc_fence_after();
-#pragma unroll
-          for (int dy = 0; dy < 3; ++dy) {
-            const unsigned xr = xbase + (unsigned)(((L0 + i + dy) % NROW) * ROW_BYTES);
-            const unsigned gr = gbase + (unsigned)(qg * WG_G_BYTES);
-            for (int k = 0; k < ksteps; ++k)
-              mma_f16_wg(tmem + (unsigned)(dy * HC), smem_desc_mn_sw64(xr + (unsigned)(k * 16 * PIX_BYTES), PIX_BYTES),
-                         smem_desc_mn_sw64(gr + (unsigned)(k * 16 * PIX_BYTES), PIX_BYTES),
-                         (T > 0 || k > 0) ? 1u : 0u);
+      /* accumulators [blk, blk + cnt) += A B */
+      auto mma = [&](unsigned long long ad, unsigned gr, int blk, int cnt) {
+        mma_f16(tmem + (unsigned)(blk * HC), ad, smem_desc_mn_sw64(gr, WG_G_BYTES), idesc(cnt) | kMnMajor, 1u);
+      };
+      /* only MMAs of one shape and accumulator are pipelined in order: where
+       * the accumulators' split changes, the MMAs of the last input row come
+       * first (its slot's release) */
+      int split = 0, last = 0; /* the last ring slot released by a commit */
+      auto same_split = [&](int s) {
+        const bool wait = split != 0 && split != s;
+        split = s;
+        return !wait || bar_wait(&xempty[last % WG_NX], (last / WG_NX) & 1);
+      };
+      for (int t = blockIdx.x; t < n.total && ok; t += gridDim.x) {
+        const Item it = item_at(t, n);
+        if (it.tail) {
+          if (L & 1) {
+            if (!(ok = xlanded(L))) break;
+            bar_arrive(&xempty[L % WG_NX]);
+            ++L;
           }
-          mma_commit(&xempty[(L0 + i) % NROW]);  /* input row y - 1 is read for the last time */
-          mma_commit(&gempty[qg]);
+          if (!(ok = xlanded(L) && xlanded(L + 1) && glanded(G) && same_split(1 << 8))) break;
+          tc_fence_after();
+          const unsigned xr = xbase + (unsigned)((L % WG_NX) * ROW_BYTES);
+          const unsigned gr = gbase + (unsigned)((G % WG_NG) * WG_G_BYTES);
+          for (int dy = 0; dy < 3; ++dy)
+            for (int k = 0; k < BAND / 2; ++k) /* two rows of 8 pixels per K of 16 */
+              mma(smem_desc_mn_sw64(xr + (unsigned)((2 * k + dy) * TAIL_PITCH), PIX_BYTES, TAIL_PITCH),
+                  gr + (unsigned)(2 * k * TAIL_W * PIX_BYTES), 2 - dy, 1);
+          mma_commit(&xempty[L % WG_NX]);
+          mma_commit(&xempty[(L + 1) % WG_NX]);
+          mma_commit(&gempty[G % WG_NG]);
+          last = L + 1;
+          L += 2;
+          ++G;
+          continue;
         }
-        if (!ok) break;
-        mma_commit(&xempty[(L0 + it.rows) % NROW]);
-        mma_commit(&xempty[(L0 + it.rows + 1) % NROW]);
-        L0 += it.rows + 2;
-        G0 += it.rows;
+        /* K blocks holding pixels of the image: past it the gradient is zero */
+        const int ksteps = (n.W - it.x0 >= TM) ? TM / 16 : (n.W - it.x0 + 15) / 16;
+        for (int j = 0; j < it.rows + 2 && ok; ++j, ++L) {
+          /* input row j meets gradient rows lo .. hi of the band, row i for kernel row j - i */
+          const int lo = j > 2 ? j - 2 : 0, hi = j < it.rows ? j : it.rows - 1;
+          const int room = WG_NG - (G + lo) % WG_NG, cnt = hi - lo + 1;
+          const int c0 = cnt < room ? cnt : room;
+          const int blk = 2 - (j - lo);
+          ok = xlanded(L) && (j >= it.rows || glanded(G + j)) && same_split(1 + blk + 4 * c0 + 16 * cnt);
+          if (!ok) break;
+          tc_fence_after();
+          const unsigned xr = xbase + (unsigned)((L % WG_NX) * ROW_BYTES);
+          const unsigned g0 = gbase + (unsigned)(((G + lo) % WG_NG) * WG_G_BYTES);
+          for (int k = 0; k < ksteps; ++k) {
+            const unsigned off = (unsigned)(k * 16 * PIX_BYTES);
+            const unsigned long long ad = smem_desc_mn_sw64(xr + off, PIX_BYTES);
+            mma(ad, g0 + off, blk, c0);
+            if (c0 < cnt) mma(ad, gbase + off, blk + c0, cnt - c0); /* the ring of gradient rows wraps */
+          }
+          mma_commit(&xempty[L % WG_NX]);
+          last = L;
+          if (j >= 2) mma_commit(&gempty[(G + j - 2) % WG_NG]); /* read for the last time */
+        }
+        G += it.rows;
       }
       if (!ok) atomicExch(&abort_flag, 1);
       mma_commit(done); /* arrives once every MMA issued above has completed */
     }
   } else {
+    /* ---- bias sums: thread = 16-byte chunk (8 channels) of every 32nd pixel
+     * of each staged gradient row (zero outside the image) */
+    float sum[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum[k] = 0.f;
+    const int chunk = tid & 3;
+    int G = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < n.total && ok; t += gridDim.x) {
+      const int count = item_at(t, n).tiles();
+      for (int i = 0; i < count; ++i, ++G) {
+        ok = bar_wait(&gfull[G % WG_NG], (G / WG_NG) & 1) && !*(volatile int*)&abort_flag;
+        ok = !__any_sync(0xffffffffu, !ok);
+        if (!ok) break;
+        const unsigned char* row = grows + (G % WG_NG) * WG_G_BYTES;
+#pragma unroll
+        for (int r = 0; r < TM / 32; ++r) {
+          const int px = (tid >> 2) + 32 * r;
+          const uint4 v = *reinterpret_cast<const uint4*>(row + px * PIX_BYTES + ((chunk ^ ((px >> 1) & 3)) << 4));
+          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 f = __bfloat1622float2(h[k]);
+            sum[2 * k] += f.x;
+            sum[2 * k + 1] += f.y;
+          }
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(&gempty[G % WG_NG]);
+      }
+    }
+    if (!ok) atomicExch(&abort_flag, 1);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+      if (lane < 4) bias_sum[warp][chunk * 8 + k] = sum[k];
+    }
     /* ---- epilogue: warp w reads TMEM lanes 32 w .. (shift j = w, channel
      * ci = lane) of each kernel row's accumulator */
-    const bool ok = bar_wait(done, 0);
-    if (__any_sync(0xffffffffu, !ok)) atomicExch(&abort_flag, 1);
-    if (ok && !*(volatile int*)&abort_flag && warp < 3) {
+    const bool fin = bar_wait(done, 0);
+    if (__any_sync(0xffffffffu, !fin)) atomicExch(&abort_flag, 1);
+    asm volatile("bar.sync 1, 128;" ::: "memory"); /* the bias sums of the four warps */
+    if (!__any_sync(0xffffffffu, !fin || *(volatile int*)&abort_flag)) {
       /* the grid never exceeds the items, so every CTA accumulated rows */
-      float* out = partial + (long long)blockIdx.x * 9 * HC * HC;
+      float* out = partial + (long long)blockIdx.x * WG_PART;
+      if (warp < 3) {
 #pragma unroll
-      for (int dy = 0; dy < 3; ++dy) {
-        float v[32];
-        tc_fence_after();
-        tmem_ld32(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(dy * HC), v);
-        const int tap = dy * 3 + warp;
+        for (int dy = 0; dy < 3; ++dy) {
+          float v[32];
+          tc_fence_after();
+          tmem_ld32(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)((2 - dy) * HC), v);
+          const int tap = dy * 3 + warp;
 #pragma unroll
-        for (int co = 0; co < HC; ++co) out[(tap * HC + co) * HC + lane] = v[co];
+          for (int co = 0; co < HC; ++co) out[(tap * HC + co) * HC + lane] = v[co];
+        }
+      } else {
+        out[9 * HC * HC + lane] = (bias_sum[0][lane] + bias_sum[1][lane]) + (bias_sum[2][lane] + bias_sum[3][lane]);
       }
     }
   }
@@ -599,7 +808,7 @@ __global__ void __launch_bounds__(WG_THREADS, 2) mid_wgrad_tc(const __grid_const
   if (abort_flag) {
     if (tid == 0) atomicExch(&g_cnn_tc_status, 1);
     if (warp == WG_TMA_WARP && lane == 0) {
-      for (int j = xl_waited; j < xl_issued; ++j) bar_wait(&xfull[j % NROW], (j / NROW) & 1);
+      for (int j = xl_waited; j < xl_issued; ++j) bar_wait(&xfull[j % WG_NX], (j / WG_NX) & 1);
       for (int j = gl_waited; j < gl_issued; ++j) bar_wait(&gfull[j % WG_NG], (j / WG_NG) & 1);
     }
     if (warp == WG_MMA_WARP && lane == 0) bar_wait(done, 0);
@@ -628,18 +837,20 @@ int launch(const void* x, const void* w, const float* bias, const void* mask, vo
   /* x as [B][H][W][32]: dims innermost first */
   const unsigned long long dims[4] = {32, (unsigned long long)W, (unsigned long long)H, (unsigned long long)B};
   const unsigned long long strides[3] = {64, 64ull * W, 64ull * W * H};
-  const unsigned box[4] = {32, SEG, 1, 1};
-  CUtensorMap map;
+  const unsigned box[4] = {32, SEG, 1, 1}, tail[4] = {32, TAIL_SEG, BAND + 2, 1};
+  CUtensorMap map, tmap;
   int rc = prml_tensor_map_tiled(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, x, dims, strides, box, 64);
+  if (!rc) rc = prml_tensor_map_tiled(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, x, dims, strides, tail, 64);
   if (rc) return rc;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long items = (long long)B * ((H + BAND - 1) / BAND) * ((W + TM - 1) / TM);
-  if (items > 0x7fffffffLL) return prml_set_error(PRML_ERR_ARG, "mid_conv_tc: too many work items");
-  const int grid = (int)(items < 2LL * sms ? items : 2LL * sms);
+  if ((long long)B * H * ((W + TM - 1) / TM) > 0x7fffffffLL)
+    return prml_set_error(PRML_ERR_ARG, "mid_conv_tc: too many work items");
+  const Items n = make_items(B, H, W, band_rows(B, H, W, 2 * sms));
+  const int grid = n.total < 2 * sms ? n.total : 2 * sms;
   mid_conv_tc<MODE><<<grid, THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
-      map, static_cast<const bf16*>(w), bias, static_cast<const bf16*>(mask), static_cast<bf16*>(y), B, H, W);
+      map, tmap, static_cast<const bf16*>(w), bias, static_cast<const bf16*>(mask), static_cast<bf16*>(y), n);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return prml_set_error(PRML_ERR_CUDA, std::string("mid_conv_tc: ") + cudaGetErrorString(e));
   return PRML_OK;
@@ -659,21 +870,23 @@ int launch_wgrad(const void* x, const void* g, float* partial, int parts, int* u
   const unsigned long long strides[3] = {64, 64ull * W, 64ull * W * H};
   const unsigned xbox[4] = {32, SEG, 1, 1};
   const unsigned gbox[4] = {32, TM, 1, 1};
-  CUtensorMap xmap, gmap;
+  const unsigned xtbox[4] = {32, TAIL_SEG, BAND + 2, 1}, gtbox[4] = {32, TAIL_W, BAND, 1};
+  CUtensorMap xmap, gmap, xtail, gtail;
   int rc = prml_tensor_map_tiled(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, x, dims, strides, xbox, 64);
-  if (rc) return rc;
-  rc = prml_tensor_map_tiled(&gmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, g, dims, strides, gbox, 64);
+  if (!rc) rc = prml_tensor_map_tiled(&gmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, g, dims, strides, gbox, 64);
+  if (!rc) rc = prml_tensor_map_tiled(&xtail, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, x, dims, strides, xtbox, 64);
+  if (!rc) rc = prml_tensor_map_tiled(&gtail, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, g, dims, strides, gtbox, 64);
   if (rc) return rc;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long items = (long long)B * ((H + BAND - 1) / BAND) * ((W + TM - 1) / TM);
-  if (items > 0x7fffffffLL) return prml_set_error(PRML_ERR_ARG, "mid_wgrad_tc: too many work items");
-  long long grid = 2LL * sms;
-  if (grid > parts) grid = parts;
-  if (grid > items) grid = items;
-  *used = (int)grid;
-  mid_wgrad_tc<<<(int)grid, WG_THREADS, WG_SMEM, static_cast<cudaStream_t>(stream)>>>(xmap, gmap, partial, B, H, W);
+  if ((long long)B * H * ((W + TM - 1) / TM) > 0x7fffffffLL)
+    return prml_set_error(PRML_ERR_ARG, "mid_wgrad_tc: too many work items");
+  int grid = parts < 2 * sms ? parts : 2 * sms;
+  const Items n = make_items(B, H, W, band_rows(B, H, W, grid));
+  if (grid > n.total) grid = n.total;
+  *used = grid;
+  mid_wgrad_tc<<<grid, WG_THREADS, WG_SMEM, static_cast<cudaStream_t>(stream)>>>(xmap, gmap, xtail, gtail, partial, n);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return prml_set_error(PRML_ERR_CUDA, std::string("mid_wgrad_tc: ") + cudaGetErrorString(e));
   return PRML_OK;
