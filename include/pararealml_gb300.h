@@ -375,6 +375,12 @@ int prml_pr_update_norm(const double* new_pts, const double* old_pts, int slices
  * prml_cnn_pack_mid: forward [9][co][ci], dgrad [9][ci][co] with flipped
  * taps.  `parts` is the number of CTAs (and partial sums) of a reduction;
  * `scratch` is caller memory of the size the *_scratch_elems functions give. */
+/* The whole forward pass y = residual + s_out * net(s_in * u) with the layer
+ * functions below: params the flat float32 parameters (w0, b0, .., w5, b5),
+ * wf the four packed middle layers, acts five activations [B][H][W][32]. */
+int prml_cnn_forward(const void* u, const void* residual, void* y, int elem_bytes, int pitch, const float* params,
+                     const float* s_in, const float* s_out, const void* wf, void* acts, int B, int H, int W,
+                     void* stream);
 int prml_cnn_in_fwd(const void* u, int elem_bytes, int pitch, const float* w0, const float* b0,
                     const float* s_in, void* x1, int B, int H, int W, void* stream);
 int prml_cnn_mid_fwd(const void* x, const void* wf, const float* bias, void* y, int B, int H, int W,

@@ -120,6 +120,7 @@ def _declare(lib: ctypes.CDLL) -> None:
             _c_int,
             [_p, _p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _p, _p, _p],
         ),
+        "prml_cnn_forward": (_c_int, [_p, _p, _p, _c_int, _c_int, _p, _p, _p, _p, _p, _c_int, _c_int, _c_int, _p]),
         "prml_cnn_in_fwd": (_c_int, [_p, _c_int, _c_int, _p, _p, _p, _p, _c_int, _c_int, _c_int, _p]),
         "prml_cnn_mid_fwd": (_c_int, [_p, _p, _p, _p, _c_int, _c_int, _c_int, _p]),
         "prml_cnn_out_fwd": (_c_int, [_p, _p, _p, _p, _p, _p, _c_int, _c_int, _c_int, _c_int, _c_int, _p]),
@@ -194,6 +195,7 @@ def exported_symbols() -> list:
         "prml_pr_norm_scratch_elems",
         "prml_pr_update_norm",
         "prml_pr_update_norm_noalloc",
+        "prml_cnn_forward",
         "prml_cnn_in_fwd",
         "prml_cnn_mid_fwd",
         "prml_cnn_out_fwd",

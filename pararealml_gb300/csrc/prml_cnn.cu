@@ -264,12 +264,19 @@ __global__ void __launch_bounds__(288) mid_wgrad(const bf16* __restrict__ x, con
     }
 }
 
+/* Kernels launched by prml_launch_overlapped begin with this. */
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 /* out[i] = scale * sum_k partial[k * n + i]: a (32, 8) block per 32 outputs,
  * row ty sums the parts k = ty (mod 8), then the 8 row sums are added in
  * order (deterministic for a given part count). */
 __global__ void __launch_bounds__(256) reduce_parts(const float* __restrict__ partial, int parts, int n,
                                                     float* __restrict__ out, float scale) {
   __shared__ float red[8][32];
+  after_previous();
   const int i = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
   if (i < n)
@@ -291,6 +298,7 @@ __global__ void __launch_bounds__(256) reduce_wgrad(const float* __restrict__ pa
                                                     float* __restrict__ dw, float* __restrict__ db) {
   constexpr int n = 9 * HC * HC + HC;
   __shared__ float red[8][32];
+  after_previous();
   const int i = blockIdx.x * 32 + threadIdx.x; /* n is a multiple of 32 */
   float s = 0.f;
   for (int k = threadIdx.y; k < parts; k += 8) s += partial[(long long)k * n + i];
@@ -355,6 +363,7 @@ __global__ void __launch_bounds__(256, 2) in_fwd(const S* __restrict__ u, int pi
                                                  bf16* __restrict__ x1, int B, int H, int W) {
   __shared__ __align__(16) float ws[9 * 2 * HC + HC];
   __shared__ float us[2][TL_TR + 2][TL_TW + 2];
+  after_previous();
   for (int i = threadIdx.x; i < 9 * 2 * HC; i += blockDim.x) ws[i] = w0[i] * s_in[(i / HC) & 1];
   for (int i = threadIdx.x; i < HC; i += blockDim.x) ws[9 * 2 * HC + i] = b0[i];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -425,6 +434,7 @@ __global__ void __launch_bounds__(OUTF_THREADS) out_fwd(const bf16* __restrict__
                                                         int B, int H, int W) {
   __shared__ __align__(16) float ws[9 * HC * 2];
   __shared__ __align__(16) bf16 xs[(OUTF_TR + 2) * (OUTF_TW + 2) * OUTF_PS];
+  after_previous();
   for (int i = threadIdx.x; i < 9 * HC * 2; i += blockDim.x) ws[i] = w5[i];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lx = lane & 15, ly = 2 * warp + (lane >> 4);
@@ -489,6 +499,7 @@ __global__ void __launch_bounds__(256, 2) out_dgrad(const float* __restrict__ dy
                                                     bf16* __restrict__ dx5, int B, int H, int W) {
   __shared__ __align__(16) float ws[9 * HC * 2];
   __shared__ float gs[2][TL_TR + 2][TL_TW + 2];
+  after_previous();
   for (int i = threadIdx.x; i < 9 * HC * 2; i += blockDim.x) ws[i] = w5[i] * s_out[i & 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ntx = (W + TL_TW - 1) / TL_TW, nty = (H + TL_TR - 1) / TL_TR;
@@ -605,6 +616,7 @@ __global__ void __launch_bounds__(256) thin_wgrad(const bf16* __restrict__ g1, c
   __shared__ __align__(16) bf16 s32[OUT ? S_ELEMS : A_ELEMS];
   __shared__ float s2[OUT ? A_ELEMS : S_ELEMS];
   __shared__ float red[4][NK];
+  after_previous();
   const float* sa2 = s2;
   const float* ss2 = s2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -764,8 +776,9 @@ int grid_tiles(int B, int H, int W, int tr, int tw) {
   return (int)(g < 1 ? 1 : g);
 }
 
-int last(const char* what) {
-  cudaError_t e = cudaGetLastError();
+int last(const char* what, cudaError_t e = cudaSuccess) {
+  const cudaError_t sticky = cudaGetLastError();
+  if (e == cudaSuccess) e = sticky;
   return e == cudaSuccess ? PRML_OK : prml_set_error(PRML_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -787,19 +800,42 @@ bool check_dims(int B, int H, int W) { return B >= 1 && H >= 1 && W >= 1; }
 
 extern "C" {
 
+/* The whole forward pass, one host call: the six launches that the layer
+ * functions below make one by one. */
+int prml_cnn_forward(const void* u, const void* residual, void* y, int elem_bytes, int pitch, const float* params,
+                     const float* s_in, const float* s_out, const void* wf, void* acts, int B, int H, int W,
+                     void* stream) {
+  if (!params || !wf || !acts || !check_dims(B, H, W))
+    return prml_set_error(PRML_ERR_ARG, "prml_cnn_forward: bad argument");
+  constexpr int MID = 4, NW0 = 9 * 2 * HC, NWM = 9 * HC * HC;
+  const float* w0 = params;
+  const float* mid = w0 + NW0 + HC;                     /* w1, b1, .., w4, b4 */
+  const float* w5 = mid + (long long)MID * (NWM + HC);
+  const long long act = (long long)B * H * W * HC;
+  bf16* a = static_cast<bf16*>(acts);
+  int rc = prml_cnn_in_fwd(u, elem_bytes, pitch, w0, w0 + NW0, s_in, a, B, H, W, stream);
+  for (int l = 0; l < MID && !rc; ++l)
+    rc = prml_cnn_mid_fwd(a + l * act, static_cast<const bf16*>(wf) + l * NWM, mid + l * (NWM + HC) + NWM,
+                          a + (l + 1) * act, B, H, W, stream);
+  if (rc) return rc;
+  return prml_cnn_out_fwd(a + MID * act, w5, w5 + 9 * HC * 2, s_out, residual, y, elem_bytes, pitch, B, H, W, stream);
+}
+
 int prml_cnn_in_fwd(const void* u, int elem_bytes, int pitch, const float* w0, const float* b0,
                     const float* s_in, void* x1, int B, int H, int W, void* stream) {
   if (!u || !w0 || !b0 || !s_in || !x1 || !check_dims(B, H, W) || pitch < W)
     return prml_set_error(PRML_ERR_ARG, "prml_cnn_in_fwd: bad argument");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaSuccess;
   const int g = grid_tiles(B, H, W, TL_TR, TL_TW);
   if (elem_bytes == 4)
-    in_fwd<float><<<g, 256, 0, s>>>(static_cast<const float*>(u), pitch, w0, b0, s_in, static_cast<bf16*>(x1), B, H, W);
+    e = prml_launch_overlapped(in_fwd<float>, g, dim3(256), 0, stream, static_cast<const float*>(u), pitch, w0, b0, s_in,
+                               static_cast<bf16*>(x1), B, H, W);
   else if (elem_bytes == 8)
-    in_fwd<double><<<g, 256, 0, s>>>(static_cast<const double*>(u), pitch, w0, b0, s_in, static_cast<bf16*>(x1), B, H, W);
+    e = prml_launch_overlapped(in_fwd<double>, g, dim3(256), 0, stream, static_cast<const double*>(u), pitch, w0, b0, s_in,
+                               static_cast<bf16*>(x1), B, H, W);
   else
     return prml_set_error(PRML_ERR_ARG, "prml_cnn_in_fwd: elem_bytes must be 4 or 8");
-  return last("prml_cnn_in_fwd");
+  return last("prml_cnn_in_fwd", e);
 }
 
 int prml_cnn_mid_fwd(const void* x, const void* wf, const float* bias, void* y, int B, int H, int W,
@@ -845,8 +881,8 @@ int prml_cnn_mid_wgrad(const void* x, const void* g, float* dw, float* db, int p
     int used = parts;
     rc = prml_cnn_mid_wgrad_tc(x, g, scratch, parts, &used, B, H, W, stream);
     if (rc) return rc;
-    reduce_wgrad<<<9 * HC + 1, dim3(32, 8), 0, s>>>(scratch, used, dw, db);
-    return last("prml_cnn_mid_wgrad");
+    const cudaError_t e = prml_launch_overlapped(reduce_wgrad, 9 * HC + 1, dim3(32, 8), 0, stream, scratch, used, dw, db);
+    return last("prml_cnn_mid_wgrad", e);
   }
   mid_wgrad<<<parts, 288, WG_SMEM, s>>>(static_cast<const bf16*>(x), static_cast<const bf16*>(g), scratch, B, H, W);
   reduce_parts<<<(n + 31) / 32, dim3(32, 8), 0, s>>>(scratch, parts, n, co_major, 1.f);
@@ -861,17 +897,17 @@ int prml_cnn_out_fwd(const void* x5, const float* w5, const float* b5, const flo
                      void* stream) {
   if (!x5 || !w5 || !b5 || !s_out || !u || !y || !check_dims(B, H, W) || pitch < W)
     return prml_set_error(PRML_ERR_ARG, "prml_cnn_out_fwd: bad argument");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaSuccess;
   const int g = grid_tiles(B, H, W, OUTF_TR, OUTF_TW);
   if (elem_bytes == 4)
-    out_fwd<float><<<g, OUTF_THREADS, 0, s>>>(static_cast<const bf16*>(x5), w5, b5, s_out, static_cast<const float*>(u),
-                                     static_cast<float*>(y), pitch, B, H, W);
+    e = prml_launch_overlapped(out_fwd<float>, g, dim3(OUTF_THREADS), 0, stream, static_cast<const bf16*>(x5), w5, b5, s_out,
+                               static_cast<const float*>(u), static_cast<float*>(y), pitch, B, H, W);
   else if (elem_bytes == 8)
-    out_fwd<double><<<g, OUTF_THREADS, 0, s>>>(static_cast<const bf16*>(x5), w5, b5, s_out, static_cast<const double*>(u),
-                                      static_cast<double*>(y), pitch, B, H, W);
+    e = prml_launch_overlapped(out_fwd<double>, g, dim3(OUTF_THREADS), 0, stream, static_cast<const bf16*>(x5), w5, b5, s_out,
+                               static_cast<const double*>(u), static_cast<double*>(y), pitch, B, H, W);
   else
     return prml_set_error(PRML_ERR_ARG, "prml_cnn_out_fwd: elem_bytes must be 4 or 8");
-  return last("prml_cnn_out_fwd");
+  return last("prml_cnn_out_fwd", e);
 }
 
 int prml_cnn_out_bwd(const float* dy, const void* x5, const float* w5, const float* s_out, void* dx5,

@@ -97,6 +97,11 @@ __device__ __forceinline__ constexpr unsigned idesc(int blocks) {
 
 __device__ int g_cnn_tc_status;
 
+/* The next launch may start once every CTA of this one has got its tensor
+ * memory; nothing global is touched before the previous launch is complete. */
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ unsigned saddr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -293,13 +298,6 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  /* weights [dy][dx][n][k] -> [dx][chunk][2 - dy][n][8], bias */
-  for (int i = tid; i < 9 * HC * 4; i += THREADS) {
-    const int tap = i / (HC * 4), rem = i - tap * HC * 4, co = rem >> 2, c = rem & 3;
-    const uint4 v = *reinterpret_cast<const uint4*>(w + (tap * HC + co) * HC + c * 8);
-    *reinterpret_cast<uint4*>(wsm + (((tap % 3) * 4 + c) * 3 * HC + (2 - tap / 3) * HC + co) * 16) = v;
-  }
-  if (MODE == 0 && tid < HC) bias_s[tid] = bias[tid];
   if (tid == 0) {
     for (int s = 0; s < NROW; ++s) {
       bar_init(&full[s], 1);
@@ -315,8 +313,6 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
     loads_waited = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  /* generic-proxy weight stores must be visible to the tensor cores */
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tmem_slot)),
                  "r"(TMEM_COLS)
@@ -329,6 +325,18 @@ __global__ void __launch_bounds__(THREADS, 2) mid_conv_tc(const __grid_constant_
   const unsigned tmem = *tmem_slot;
   if (warp < 4)
     for (int a = 0; a < NACC; ++a) tmem_zero32(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(a * HC));
+  let_next_start();
+  wait_previous();
+
+  /* weights [dy][dx][n][k] -> [dx][chunk][2 - dy][n][8], bias */
+  for (int i = tid; i < 9 * HC * 4; i += THREADS) {
+    const int tap = i / (HC * 4), rem = i - tap * HC * 4, co = rem >> 2, c = rem & 3;
+    const uint4 v = *reinterpret_cast<const uint4*>(w + (tap * HC + co) * HC + c * 8);
+    *reinterpret_cast<uint4*>(wsm + (((tap % 3) * 4 + c) * 3 * HC + (2 - tap / 3) * HC + co) * 16) = v;
+  }
+  if (MODE == 0 && tid < HC) bias_s[tid] = bias[tid];
+  /* generic-proxy weight stores must be visible to the tensor cores */
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -608,6 +616,8 @@ __global__ void __launch_bounds__(WG_THREADS, 2) mid_wgrad_tc(const __grid_const
   const unsigned tmem = tmem_slot;
   if (warp < 4)
     for (int a = 0; a < 3; ++a) tmem_zero32(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(a * HC));
+  let_next_start();
+  wait_previous();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -849,9 +859,9 @@ int launch(const void* x, const void* w, const float* bias, const void* mask, vo
     return prml_set_error(PRML_ERR_ARG, "mid_conv_tc: too many work items");
   const Items n = make_items(B, H, W, band_rows(B, H, W, 2 * sms));
   const int grid = n.total < 2 * sms ? n.total : 2 * sms;
-  mid_conv_tc<MODE><<<grid, THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
-      map, tmap, static_cast<const bf16*>(w), bias, static_cast<const bf16*>(mask), static_cast<bf16*>(y), n);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = prml_launch_overlapped(mid_conv_tc<MODE>, grid, dim3(THREADS), SMEM_BYTES, stream, map, tmap,
+                                               static_cast<const bf16*>(w), bias, static_cast<const bf16*>(mask),
+                                               static_cast<bf16*>(y), n);
   if (e != cudaSuccess) return prml_set_error(PRML_ERR_CUDA, std::string("mid_conv_tc: ") + cudaGetErrorString(e));
   return PRML_OK;
 }
@@ -886,8 +896,8 @@ int launch_wgrad(const void* x, const void* g, float* partial, int parts, int* u
   const Items n = make_items(B, H, W, band_rows(B, H, W, grid));
   if (grid > n.total) grid = n.total;
   *used = grid;
-  mid_wgrad_tc<<<grid, WG_THREADS, WG_SMEM, static_cast<cudaStream_t>(stream)>>>(xmap, gmap, xtail, gtail, partial, n);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = prml_launch_overlapped(mid_wgrad_tc, grid, dim3(WG_THREADS), WG_SMEM, stream, xmap, gmap, xtail,
+                                               gtail, partial, n);
   if (e != cudaSuccess) return prml_set_error(PRML_ERR_CUDA, std::string("mid_wgrad_tc: ") + cudaGetErrorString(e));
   return PRML_OK;
 }

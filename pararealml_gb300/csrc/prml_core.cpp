@@ -416,6 +416,8 @@ int prml_set_step_overlap(int enabled) {
   return prev;
 }
 
+int prml_step_overlap() { return g_step_overlap; }
+
 static int launch_step(Kernel* k, int block, int grid, prml_step_params* p, void* second,
                        CUstream stream, void* third = nullptr) {
   void* args[] = {p, second, third};

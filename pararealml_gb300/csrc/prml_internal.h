@@ -3,6 +3,7 @@
 #define PRML_INTERNAL_H
 
 #include <cuda.h>
+#include <cuda_runtime.h>
 
 #include <string>
 
@@ -10,6 +11,27 @@
 
 /* Records `msg` as the calling thread's last error and returns `code`. */
 int prml_set_error(int code, const std::string& msg);
+
+/* Whether launches may overlap their predecessor (prml_set_step_overlap). */
+extern "C" int prml_step_overlap();
+
+/* Launches a kernel that waits (griddepcontrol.wait) before it touches global
+ * memory, so that its start overlaps the end of its predecessor in the stream
+ * (programmatic dependent launch). */
+template <typename... P, typename... A>
+cudaError_t prml_launch_overlapped(void (*kernel)(P...), int grid, dim3 block, size_t smem, void* stream, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = attr;
+  cfg.numAttrs = prml_step_overlap() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 /* The calling thread's current CUDA context (driver handle), or NULL. */
 void* prml_current_context();

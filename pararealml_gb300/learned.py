@@ -150,20 +150,16 @@ class ResidualCNN:
     def forward(self, u, y, H: int, W: int, residual=None) -> None:
         """y = r + s_out * net(s_in * u) with r = ``residual`` (default u);
         u, y, r planar device states (B, 2, H, pitch)."""
-        lib = _native.lib()
-        B, pitch, es = u.shape[0], u.shape[-1], u.element_size()
-        ws = self._ws(B, H, W)
-        acts = ws["acts"]
-        s = _stream()
-        chk = _native.check
-        chk(lib.prml_cnn_in_fwd(u.data_ptr(), es, pitch, self.w(0).data_ptr(), self.b(0).data_ptr(),
-                                self.s_in.data_ptr(), acts[0].data_ptr(), B, H, W, s), "cnn in")
-        for i in range(N_MID):
-            chk(lib.prml_cnn_mid_fwd(acts[i].data_ptr(), self.wf[i].data_ptr(), self.b(i + 1).data_ptr(),
-                                     acts[i + 1].data_ptr(), B, H, W, s), "cnn mid")
-        chk(lib.prml_cnn_out_fwd(acts[N_MID].data_ptr(), self.w(LAYERS - 1).data_ptr(), self.b(LAYERS - 1).data_ptr(),
-                                 self.s_out.data_ptr(), (u if residual is None else residual).data_ptr(), y.data_ptr(),
-                                 es, pitch, B, H, W, s), "cnn out")
+        r = u if residual is None else residual
+        acts = self._ws(u.shape[0], H, W)["acts"]
+        _native.check(
+            _native.lib().prml_cnn_forward(
+                u.data_ptr(), r.data_ptr(), y.data_ptr(), u.element_size(), u.shape[-1], self.params.data_ptr(),
+                self.s_in.data_ptr(), self.s_out.data_ptr(), self.wf.data_ptr(), acts.data_ptr(), u.shape[0], H, W,
+                _stream(),
+            ),
+            "cnn forward",
+        )
 
     def loss_and_dy(self, y, target, H: int, W: int) -> "torch.Tensor":
         """Writes dL/dy of the mean squared error into the workspace; returns the loss (device scalar)."""
