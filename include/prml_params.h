@@ -157,6 +157,20 @@ typedef struct prml_stage_params {
   int pad;
 } prml_stage_params;
 
+/* ---- all steps of a small mesh in one launch ------------------------------
+ * Second parameter of the resident kernels: one thread-block cluster per
+ * instance keeps its state in shared memory, `band` rows per CTA. `in` is the
+ * state before the first step, `out` the first saved state, `t`, `bc_slot0`
+ * those of the first step. */
+typedef struct prml_resident_params {
+  long long n_steps;
+  long long step_stride; /* elements between saved states in `out`           */
+  int save_every;        /* n_steps is a multiple                            */
+  int band;              /* rows of the mesh per CTA                         */
+  int spitch;            /* elements between rows in shared memory, > ny + 1 */
+  int scomp;             /* elements between components there                */
+} prml_resident_params;
+
 /* ---- secant iterations of an implicit step --------------------------------
  * One launch of a generated secant kernel (MODE 2 of the step body, float64)
  * is one iteration of the reference's element-wise secant solve: the

@@ -103,6 +103,10 @@ def _declare(lib: ctypes.CDLL) -> None:
             _c_int,
             [_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _p, _p, _c_ll, _p, _c_ll, _c_ll, _p, _p, _c_ll, _c_ll, _c_int, _c_d, _c_d, _p],
         ),
+        "prml_kernel_max_cluster": (_c_int, [_p, _c_int, ctypes.POINTER(_c_int)]),
+        "prml_resident_params_size": (_c_int, []),
+        "prml_fdm_run_resident": (_c_int, [_p, _c_int, _c_int, _c_int, _c_int, _c_int, _p, _p, _c_ll, _p, _c_ll, _c_ll,
+                                           _c_ll, _c_int, _c_d, _c_d, _p]),
         "prml_stage_params_size": (_c_int, []),
         "prml_fdm_run_stages": (_c_int, [_p, _c_int, _c_int, _p, _c_int, _p, _c_ll, _p, _c_ll, _c_ll, _p, _p, _c_ll,
                                          _p, _p, _p, _c_ll, _c_int, _c_d, _c_d, _p]),
@@ -182,6 +186,9 @@ def exported_symbols() -> list:
         "prml_kernel_occupancy",
         "prml_fdm_run",
         "prml_fdm_rhs",
+        "prml_kernel_max_cluster",
+        "prml_resident_params_size",
+        "prml_fdm_run_resident",
         "prml_stage_params_size",
         "prml_fdm_run_stages",
         "prml_set_step_overlap",

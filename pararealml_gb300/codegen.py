@@ -77,6 +77,17 @@ MARCH_JOBS: Tuple[int, ...] = (4, 8, 12, 16, 20, 24)
 # 2 / 2.5, 16 x 257^2 in float64 9.1 / 10.1 / 11.4 / 11.7 ms
 MARCH_EDGE = {4: 1.5, 8: 1.0}
 MARCH_THREADS = 128
+# 2D kernels that keep a small mesh in the shared memory of a cluster: threads
+# per CTA, most vertices of an instance by element size, most shared memory of a
+# CTA.  Sixteen SMs are all an instance gets, so the float64 pipe ends the gain
+# early (us per forward Euler diffusion step, one instance, against the best
+# other kernel: 65^2 1.5 / 2.4, 97^2 2.5 / 2.4, 129^2 2.8 / 2.9 with later
+# Parareal iterations of few instances slower; float32 0.74 / 1.64, 1.1 / 1.7,
+# 1.3 / 1.7 and at 161^2 1.6 / 1.9)
+RESIDENT_THREADS = 512
+RESIDENT_VERTICES = {4: 1 << 15, 8: 10000}
+RESIDENT_SMEM = 200 << 10
+RESIDENT_TILE = (1, 1, RESIDENT_THREADS, 1, 0, "c")
 # 3D kernels launched once per integrator stage: planes per thread (97^3 RK4
 # in float64: 1, 2 and 4 planes 2.38, 2.54 and 2.64 ms per 20 steps; where a
 # step is bound by its reads more planes per thread read fewer rows)
@@ -689,6 +700,7 @@ def _side_columns(low: LoweredProblem) -> Tuple[int, bool]:
 _TEMPLATE_FILES = (
     ("csrc", "fdm_step.cuh"),
     ("csrc", "fdm_march.cuh"),
+    ("csrc", "fdm_resident.cuh"),
     ("csrc", "fdm_step3d.cuh"),
     ("include", "prml_params.h"),
 )
@@ -732,6 +744,24 @@ def is_walk(tile) -> bool:
 def is_stage(tile) -> bool:
     """Whether a tile key names a kernel launched once per integrator stage."""
     return len(tile) > 5 and tile[5] == "s"
+
+
+def is_resident(tile) -> bool:
+    """Whether a tile key names the resident kernel (resident_body)."""
+    return len(tile) > 5 and tile[5] == "c"
+
+
+def resident_shape(nx: int, ny: int, comps: int, esize: int, stages: int, max_cluster: int) -> Optional[Tuple[int, int]]:
+    """(CTAs per instance, rows per CTA) of the resident kernel, or None where
+    a mesh is too large for it (or too small for two CTAs)."""
+    if max_cluster < 2 or nx < 2 or nx * ny > RESIDENT_VERTICES[esize]:
+        return None
+    band = -(-nx // max_cluster)
+    buffers = 2 if stages == 1 else 4
+    if buffers * comps * (band + 2) * (ny + 2) * esize > RESIDENT_SMEM:
+        return None
+    cluster = -(-nx // band)
+    return (cluster, band) if cluster > 1 else None
 
 
 def is_march(tile) -> bool:
@@ -782,6 +812,8 @@ def walk_tile(rows_per_thread: int, warps: int, esize: int) -> tuple:
 def kernel_name(kind: str, dtype: str, tile) -> str:
     if is_march(tile):
         return f"prml_march_{dtype}_v{tile[6]}" + (f"_k{tile[3]}" if tile[3] > 1 else "")
+    if is_resident(tile):
+        return f"prml_resident_{dtype}"
     if is_stage(tile):
         return f"prml_stage_{dtype}_z{tile[4]}"
     if is_walk(tile):
@@ -852,6 +884,8 @@ class GeneratedModule:
     multi_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
     # secant-iteration kernel of modules with exact division: (name, smem, tile)
     secant_kernel: Tuple[str, int, tuple] = None
+    # resident kernel of 2D modules: tile -> (name, most dynamic shared memory)
+    resident_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
     # 3D kernels launched once per integrator stage: tile (1, cols, threads, 1, planes, "s") -> (name, smem)
     stage_kernels: Dict[tuple, Tuple[str, int]] = dataclasses.field(default_factory=dict)
     # marching kernels: tile (jobs per SM, cols, threads, steps, 0, "m", columns per lane) -> (name, smem)
@@ -860,12 +894,12 @@ class GeneratedModule:
     @functools.cached_property
     def kernels(self) -> Dict[tuple, Tuple[str, int]]:
         """Every step kernel: tile -> (name, dynamic shared memory)."""
-        return {**self.step_kernels, **self.march_kernels, **self.stage_kernels}
+        return {**self.step_kernels, **self.march_kernels, **self.stage_kernels, **self.resident_kernels}
 
     def box(self, tile, mode: int = 0) -> Tuple[int, int]:
         """TMA box (rows, cols) a kernel of this module stages."""
         esize = 8 if self.dtype == "f64" else 4
-        if is_march(tile) or is_stage(tile):  # no tile is staged: any box the tensor map accepts
+        if is_march(tile) or is_stage(tile) or is_resident(tile):  # no tile is staged: any box the tensor map accepts
             return 1, 16 // esize
         return region(tile, halo(self.integrator, self.invariant, mode, tile), esize)
 
@@ -918,7 +952,7 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
     if three_d and comp:
         raise NotImplementedError("compensated float32 is not available on 3D meshes")
     body = [
-        '#include "fdm_step3d.cuh"' if three_d else '#include "fdm_step.cuh"\n#include "fdm_march.cuh"',
+        '#include "fdm_step3d.cuh"' if three_d else '#include "fdm_step.cuh"\n#include "fdm_march.cuh"\n#include "fdm_resident.cuh"',
         "",
         "struct Eq {",
         f"  static constexpr int C = {low.n_comp};",
@@ -1046,6 +1080,15 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
                 f"(const prml_step_params p, const __grid_constant__ prml::TmaDesc tin) "
                 f"{{ (void)tin; prml::march_body<{ctype}, Eq, {integrator}, {vw}, {depth}, {MARCH_THREADS}>(p); }}"
             )
+    resident_kernels = {}
+    if low.x_dimension == 2 and not low.lap_idx and not comp and not exact_div:
+        name = kernel_name("resident", dtype, RESIDENT_TILE)
+        resident_kernels[RESIDENT_TILE] = (name, RESIDENT_SMEM)
+        body.append(
+            f'extern "C" __global__ void __launch_bounds__({RESIDENT_THREADS}) {name}'
+            f"(const prml_step_params p, const prml_resident_params r) "
+            f"{{ prml::resident_body<{ctype}, Eq, {integrator}, {RESIDENT_THREADS}>(p, r); }}"
+        )
     rtile = (16, 32, 128)
     rname = kernel_name("rhs", dtype, rtile)
     rsm = smem_bytes(low, integrator, invariant, rtile, esize, 1)
@@ -1092,5 +1135,6 @@ def generate_source(low: LoweredProblem, integrator: int, dtype: str, exact_div:
         n_comp=low.n_comp,
         multi_kernels=multi_kernels,
         march_kernels=march_kernels,
+        resident_kernels=resident_kernels,
         secant_kernel=secant,
     )

@@ -30,14 +30,6 @@
 
 namespace prml {
 
-/* Whether a table entry holds a value (NaN = free).  float64: tested on the
- * bits, because a comparison would take a slot of the float64 pipe, which
- * bounds the float64 kernels. */
-__device__ __forceinline__ bool is_value(float v) { return v == v; }
-__device__ __forceinline__ bool is_value(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
-  return hi < 0x7ff00000u || (hi == 0x7ff00000u && __double2loint(v) == 0);
-}
 template <typename T>
 __device__ __forceinline__ T free_value() {
   if constexpr (sizeof(T) == 4) return __int_as_float(0x7fc00000);

@@ -42,6 +42,22 @@ namespace prml {
 
 enum Integrator { FORWARD_EULER = 1, EXPLICIT_MIDPOINT = 2, RK4 = 4 };
 
+/* Whether a table entry holds a value (NaN = free).  float64: tested on the
+ * bits, because a comparison would take a slot of the float64 pipe, which
+ * bounds the float64 kernels. */
+__device__ __forceinline__ bool is_value(float v) { return v == v; }
+__device__ __forceinline__ bool is_value(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
+  return hi < 0x7ff00000u || (hi == 0x7ff00000u && __double2loint(v) == 0);
+}
+/* Whether a Neumann value is zero: its ghost vertex is the mirrored vertex, and
+ * the two float64 operations that would say so are left out (a warp of 32
+ * consecutive vertices of a narrow mesh nearly always holds a face vertex). */
+__device__ __forceinline__ bool is_zero(float v) { return v == 0.f; }
+__device__ __forceinline__ bool is_zero(double v) {
+  return (((unsigned)__double2hiint(v) & 0x7fffffffu) | (unsigned)__double2loint(v)) == 0u;
+}
+
 template <typename T>
 struct MeshC {
   T inv2d0, inv2d1, invdd0, invdd1, twod0, twod1;
@@ -53,6 +69,21 @@ struct MeshC {
   const double* c1;
   const float* c0f; /* float32 copies of c0, c1 */
   const float* c1f;
+};
+
+/* With the row and component strides of a window whose shape is known at run
+ * time only (Point<.., 0, 0>). */
+template <typename T>
+struct MeshR : MeshC<T> {
+  int spitch, scomp;
+};
+template <typename T, bool RUNTIME>
+struct MeshFor {
+  using type = MeshC<T>;
+};
+template <typename T>
+struct MeshFor<T, true> {
+  using type = MeshR<T>;
 };
 
 /* The boundary tables of half-step table `slot` (time t0 + slot dt / 2 of
@@ -122,11 +153,12 @@ struct Point {
   const T* s;
   int l;
   int gi, gj;
-  const MeshC<T>* m;
+  const typename MeshFor<T, RY == 0>::type* m;
   double time;
 
   __device__ __forceinline__ T v(int c, int di, int dj) const {
-    return s[c * RXY + l + di * RY + dj];
+    if constexpr (RY == 0) return s[c * m->scomp + l + di * m->spitch + dj];
+    else return s[c * RXY + l + di * RY + dj];
   }
   __device__ __forceinline__ T face(const T* tab, int f, int c, int k) const {
     return tab[(f * Eq::C + c) * m->flen + k];
@@ -151,22 +183,22 @@ struct Point {
     if (ka == 0) {
       if (EDGE && has_neu(0, c) && qi == 0) {
         const T g = face(m->neu, 0, c, qj);
-        if (g == g) return g;
+        if (is_value(g)) return g;
       }
       if (EDGE && has_neu(1, c) && qi == m->nx - 1) {
         const T g = face(m->neu, 1, c, qj);
-        if (g == g) return g;
+        if (is_value(g)) return g;
       }
       if constexpr (Eq::EXACT_DIV) return quot(v(c, di + 1, dj) - v(c, di - 1, dj), m->twod0, m->inv2d0);
       return (v(c, di + 1, dj) - v(c, di - 1, dj)) * m->inv2d0;
     } else {
       if (EDGE && has_neu(2, c) && qj == 0) {
         const T g = face(m->neu, 2, c, qi);
-        if (g == g) return g;
+        if (is_value(g)) return g;
       }
       if (EDGE && has_neu(3, c) && qj == m->ny - 1) {
         const T g = face(m->neu, 3, c, qi);
-        if (g == g) return g;
+        if (is_value(g)) return g;
       }
       if constexpr (Eq::EXACT_DIV) return quot(v(c, di, dj + 1) - v(c, di, dj - 1), m->twod1, m->inv2d1);
       return (v(c, di, dj + 1) - v(c, di, dj - 1)) * m->inv2d1;
@@ -175,6 +207,11 @@ struct Point {
   template <int c, int ka> __device__ __forceinline__ T grad() const {
     return grad_at<c, ka, false>(0, 0);
   }
+
+  /* Register windows (RY = VW + 2) test their Neumann values without a branch
+   * on zero: with it a 1025^2 float64 step of the register-window kernel is 2 %
+   * slower, while staged float64 steps of small meshes are a quarter faster. */
+  static constexpr bool kWindow = RY > 0 && RY <= 8;
 
   /* Neighbours (prev, next) of the vertex along one kernel axis, with the
    * Neumann ghost vertices y[1] - 2dx g (lower face) and y[n-2] + 2dx g
@@ -187,20 +224,36 @@ struct Point {
     if (ka == 0) {
       if (EDGE && has_neu(0, c) && gi == 0) {
         const T g = face(m->neu, 0, c, gj);
-        if (g == g) prev = hi - m->twod0 * g;
+        if constexpr (kWindow) {
+          if (g == g) prev = hi - m->twod0 * g;
+        } else if (is_value(g)) {
+          prev = is_zero(g) ? hi : hi - m->twod0 * g;
+        }
       }
       if (EDGE && has_neu(1, c) && gi == m->nx - 1) {
         const T g = face(m->neu, 1, c, gj);
-        if (g == g) next = lo + m->twod0 * g;
+        if constexpr (kWindow) {
+          if (g == g) next = lo + m->twod0 * g;
+        } else if (is_value(g)) {
+          next = is_zero(g) ? lo : lo + m->twod0 * g;
+        }
       }
     } else {
       if (EDGE && has_neu(2, c) && gj == 0) {
         const T g = face(m->neu, 2, c, gi);
-        if (g == g) prev = hi - m->twod1 * g;
+        if constexpr (kWindow) {
+          if (g == g) prev = hi - m->twod1 * g;
+        } else if (is_value(g)) {
+          prev = is_zero(g) ? hi : hi - m->twod1 * g;
+        }
       }
       if (EDGE && has_neu(3, c) && gj == m->ny - 1) {
         const T g = face(m->neu, 3, c, gi);
-        if (g == g) next = lo + m->twod1 * g;
+        if constexpr (kWindow) {
+          if (g == g) next = lo + m->twod1 * g;
+        } else if (is_value(g)) {
+          next = is_zero(g) ? lo : lo + m->twod1 * g;
+        }
       }
     }
   }
@@ -270,19 +323,19 @@ __device__ __forceinline__ T dirichlet(T v, int c, int gi, int gj, const MeshC<T
   if (!EDGE) return v;
   if (has_dir<Eq>(0, c) && gi == 0) {
     const T d = m.dir[(0 * Eq::C + c) * m.flen + gj];
-    if (d == d) v = d;
+    if (is_value(d)) v = d;
   }
   if (has_dir<Eq>(1, c) && gi == m.nx - 1) {
     const T d = m.dir[(1 * Eq::C + c) * m.flen + gj];
-    if (d == d) v = d;
+    if (is_value(d)) v = d;
   }
   if (has_dir<Eq>(2, c) && gj == 0) {
     const T d = m.dir[(2 * Eq::C + c) * m.flen + gi];
-    if (d == d) v = d;
+    if (is_value(d)) v = d;
   }
   if (has_dir<Eq>(3, c) && gj == m.ny - 1) {
     const T d = m.dir[(3 * Eq::C + c) * m.flen + gi];
-    if (d == d) v = d;
+    if (is_value(d)) v = d;
   }
   return v;
 }

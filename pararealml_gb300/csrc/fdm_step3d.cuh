@@ -76,11 +76,11 @@ struct Point3 {
     const int q = ka == 0 ? q0 : (ka == 1 ? q1 : q2);
     if (has_neu(2 * ka, c) && q == 0) {
       const T gv = face(m->neu, 2 * ka, c, q0, q1, q2);
-      if (gv == gv) return gv;
+      if (is_value(gv)) return gv;
     }
     if (has_neu(2 * ka + 1, c) && q == m->n[ka] - 1) {
       const T gv = face(m->neu, 2 * ka + 1, c, q0, q1, q2);
-      if (gv == gv) return gv;
+      if (is_value(gv)) return gv;
     }
     const int e0 = ka == 0, e1 = ka == 1, e2 = ka == 2;
     if constexpr (Eq::EXACT_DIV)
@@ -97,11 +97,11 @@ struct Point3 {
     next = hi;
     if (has_neu(2 * ka, c) && g[ka] == 0) {
       const T gv = face(m->neu, 2 * ka, c, g[0], g[1], g[2]);
-      if (gv == gv) prev = Eq::FAST ? fmaT(-m->twod[ka], gv, hi) : hi - m->twod[ka] * gv;
+      if (is_value(gv)) prev = is_zero(gv) ? hi : (Eq::FAST ? fmaT(-m->twod[ka], gv, hi) : hi - m->twod[ka] * gv);
     }
     if (has_neu(2 * ka + 1, c) && g[ka] == m->n[ka] - 1) {
       const T gv = face(m->neu, 2 * ka + 1, c, g[0], g[1], g[2]);
-      if (gv == gv) next = Eq::FAST ? fmaT(m->twod[ka], gv, lo) : lo + m->twod[ka] * gv;
+      if (is_value(gv)) next = is_zero(gv) ? lo : (Eq::FAST ? fmaT(m->twod[ka], gv, lo) : lo + m->twod[ka] * gv);
     }
   }
 
@@ -155,7 +155,7 @@ __device__ __forceinline__ T dirichlet3(T v, int c, const int (&g)[3], const Mes
     const int ka = f >> 1;
     if (g[ka] != ((f & 1) ? m.n[ka] - 1 : 0)) continue;
     const T d = m.dir[(f * Eq::C + c) * m.flen + face_index3(f, g[0], g[1], g[2], m.n)];
-    if (d == d) v = d;
+    if (is_value(d)) v = d;
   }
   return v;
 }
@@ -491,9 +491,9 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
  * GB300, us per RK4 step, the best staged whole-step tile against this (both
  * fused order): 13^3 vertices 31 -> 17 in float64 and 16.5 -> 15.5 in float32,
  * 49^3 136 -> 45 and 36 -> 18, 97^3 723 -> 126 and 148 -> 26 (before the
- * fused order 967 in float64).  What bounds it: 97^3 in float64 the float64
- * pipe (about 15 instructions a vertex and stage with the faces', 22 us of
- * 33), small meshes the four dependent launches.  One-stage steps: 49^3
+ * fused order 967 in float64; 98 since faces test their values on bits).  What
+ * bounds it: 97^3 in float64 the float64 pipe (about 11 instructions a vertex
+ * and stage, 16 us of 24), small meshes the four dependent launches.  One-stage steps: 49^3
  * 4.6 -> 3.9 and 97^3 10.9 -> 6.1 in float32, 97^3 34 -> 31 in float64; 13^3
  * 3.5 -> 3.8 (the tuner keeps the staged tile there).
  *

@@ -59,6 +59,7 @@ struct Driver {
   CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
                            unsigned, CUstream, void**, void**) = nullptr;
   CUresult (*LaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr; /* optional */
+  CUresult (*OccupancyMaxActiveClusters)(int*, CUfunction, const CUlaunchConfig*) = nullptr; /* optional */
   CUresult (*TensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                    const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -91,6 +92,7 @@ bool driver() {
          bind(h, "cuLaunchKernel", d.LaunchKernel) &&
          bind(h, "cuTensorMapEncodeTiled", d.TensorMapEncodeTiled);
   bind(h, "cuLaunchKernelEx", d.LaunchKernelEx);
+  bind(h, "cuOccupancyMaxActiveClusters", d.OccupancyMaxActiveClusters);
   if (d.ok) g_drv = d;
   return d.ok;
 }
@@ -252,8 +254,11 @@ int prml_module_kernel(void* module, const char* name, int smem_bytes, void** ke
   k->smem = smem_bytes;
   /* the staged step kernels keep everything in shared memory and gain
    * nothing from L1: ask for the largest shared-memory carveout (a
-   * preference); kernels without dynamic shared memory for the largest L1 */
-  g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_PREFERRED_SHARED_MEMORY_CARVEOUT, smem_bytes > 0 ? 100 : 0);
+   * preference); kernels without dynamic shared memory for 32 KB (14 %), the
+   * 1 KB each of the 32 CTAs an SM can hold, and the rest as L1: with none
+   * asked for, 64-thread CTAs were not all resident (16 x 131^2 Cahn-Hilliard in
+   * float64: 21.8 us a step instead of 13.4) */
+  g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_PREFERRED_SHARED_MEMORY_CARVEOUT, smem_bytes > 0 ? 100 : 14);
   /* opt in to the requested dynamic size whatever it is: a kernel with
    * static shared memory too (the multi-round kernels' group tables) can
    * exceed the 48 KB default with less than 48 KB of dynamic memory */
@@ -550,6 +555,100 @@ int prml_fdm_run(void* kernel, int block, int tile_x, int tile_y, int box_rows, 
     cur_bstride = out_bstride;
     cur_map = out_map;
     cur_slot = out_slot;
+  }
+  return PRML_OK;
+}
+
+int prml_resident_params_size(void) { return (int)sizeof(prml_resident_params); }
+
+/* launch of the resident kernel: `cluster` CTAs per instance */
+static void cluster_config(CUlaunchConfig* cfg, CUlaunchAttribute* attr, int cluster, long long grid, int block, int smem,
+                           CUstream stream) {
+  std::memset(cfg, 0, sizeof(*cfg));
+  std::memset(attr, 0, sizeof(*attr));
+  attr->id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+  attr->value.clusterDim.x = (unsigned)cluster;
+  attr->value.clusterDim.y = attr->value.clusterDim.z = 1;
+  cfg->gridDimX = (unsigned)grid;
+  cfg->gridDimY = cfg->gridDimZ = 1;
+  cfg->blockDimX = (unsigned)block;
+  cfg->blockDimY = cfg->blockDimZ = 1;
+  cfg->sharedMemBytes = (unsigned)smem;
+  cfg->hStream = stream;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+
+int prml_kernel_max_cluster(void* kernel, int block, int* cluster) {
+  Kernel* k = static_cast<Kernel*>(kernel);
+  if (!k || !cluster || block < 32 || block > 1024) return fail(PRML_ERR_ARG, "prml_kernel_max_cluster: bad argument");
+  *cluster = 0;
+  if (!g_drv.LaunchKernelEx || !g_drv.OccupancyMaxActiveClusters) return PRML_OK;
+  const bool wide = g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1) == CUDA_SUCCESS;
+  for (int n = wide ? 16 : 8; n > 1; n >>= 1) {
+    CUlaunchConfig cfg;
+    CUlaunchAttribute attr;
+    cluster_config(&cfg, &attr, n, n, block, k->smem, nullptr);
+    int active = 0;
+    if (g_drv.OccupancyMaxActiveClusters(&active, k->fn, &cfg) == CUDA_SUCCESS && active > 0) {
+      *cluster = n;
+      return PRML_OK;
+    }
+  }
+  return PRML_OK;
+}
+
+int prml_fdm_run_resident(void* kernel, int block, int cluster, int band, int comps, int buffers,
+                          const prml_step_params* base, const void* y0, long long y0_bstride, void* traj,
+                          long long traj_bstride, long long traj_step_stride, long long n_steps, int save_every, double t0,
+                          double dt, void* stream) {
+  Kernel* k = static_cast<Kernel*>(kernel);
+  if (!k) return fail(PRML_ERR_ARG, "prml_fdm_run_resident: null kernel");
+  int rc = check_geometry(base, 1, 1, block);
+  if (rc) return rc;
+  if (!y0 || !traj || n_steps < 0 || save_every < 1 || comps < 1 || (buffers != 2 && buffers != 4) || band < 1 ||
+      cluster < 1 || cluster > 16 || (long long)band * cluster < base->nx || (long long)band * (cluster - 1) >= base->nx)
+    return fail(PRML_ERR_ARG, "prml_fdm_run_resident: bad buffers, bands or step counts");
+  if (n_steps % save_every != 0)
+    return fail(PRML_ERR_ARG, "prml_fdm_run_resident: n_steps must be a multiple of save_every");
+  if (!g_drv.LaunchKernelEx) return fail(PRML_ERR_CUDA, "this driver launches no clusters");
+  prml_resident_params rp;
+  std::memset(&rp, 0, sizeof(rp));
+  rp.step_stride = traj_step_stride;
+  rp.save_every = save_every;
+  rp.band = band;
+  rp.spitch = base->ny + 2;
+  const long long scomp = (long long)(band + 2) * rp.spitch;
+  const long long smem = (long long)buffers * comps * scomp * base->elem_bytes;
+  if (smem > k->smem) return fail(PRML_ERR_ARG, "prml_fdm_run_resident: the bands do not fit in shared memory");
+  rp.scomp = (int)scomp;
+  if (cluster > 8)
+    PRML_CU(g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1));
+  prml_step_params p = *base;
+  p.dt = dt;
+  p.dt_f = (float)dt;
+  p.tb_steps = 1;
+  /* a launch ends on a saved step; long runs in several launches */
+  long long chunk = 16384 / save_every * (long long)save_every;
+  if (chunk < save_every) chunk = save_every;
+  const char* cur = static_cast<const char*>(y0);
+  long long cur_bstride = y0_bstride;
+  for (long long done = 0; done < n_steps; done += chunk) {
+    rp.n_steps = n_steps - done < chunk ? n_steps - done : chunk;
+    p.in = cur;
+    p.in_bstride = cur_bstride;
+    char* out = static_cast<char*>(traj) + (size_t)(done / save_every) * traj_step_stride * base->elem_bytes;
+    p.out = out;
+    p.out_bstride = traj_bstride;
+    p.t = t0 + (double)done * dt;
+    p.bc_slot0 = base->bc_slot0 + (int)(2 * done);
+    CUlaunchConfig cfg;
+    CUlaunchAttribute attr;
+    cluster_config(&cfg, &attr, cluster, (long long)cluster * base->batch, block, (int)smem, static_cast<CUstream>(stream));
+    void* args[] = {&p, &rp};
+    PRML_CU(g_drv.LaunchKernelEx(&cfg, k->fn, args, nullptr));
+    cur = out + (size_t)(rp.n_steps / save_every - 1) * traj_step_stride * base->elem_bytes;
+    cur_bstride = traj_bstride;
   }
   return PRML_OK;
 }

@@ -254,6 +254,7 @@ class StencilPlan:
         self._tuned_ctas: Dict[bool, int] = {}  # trajectory pattern -> tuned grid cap (0 = fill the GPU)
         self._user_ctas = 0
         self._march_rows: Dict[tuple, Tuple[int, int]] = {}
+        self._resident = False  # resident_shape(), once asked for
         self.last_tile: Optional[Tuple[int, ...]] = self.tile
         self.last_ctas = 0  # grid cap of the latest run (0 = every resident CTA)
         if self.tile is not None and self.tile not in self.module.gen.kernels:
@@ -849,6 +850,21 @@ class StencilPlan:
     def _launch(self, tile, y0, y0_bstride, traj, traj_bstride, traj_step_stride, wa, wb,
                 n_steps, save_every, t0, dt) -> None:
         stage = codegen.is_stage(tile)
+        if codegen.is_resident(tile):
+            shape = self.resident_shape()
+            if shape is None:
+                raise ValueError("the mesh is too large for the resident step kernel")
+            cluster, band = shape
+            self.params.jobs_per_cta = 1
+            _native.check(
+                _native.lib().prml_fdm_run_resident(
+                    self._step_kernel(tile), tile[2], cluster, band, self.C, 2 if self._stages() == 1 else 4,
+                    ctypes.byref(self.params), y0, y0_bstride, traj, traj_bstride, traj_step_stride, n_steps, save_every,
+                    float(t0), float(dt), self.stream_handle(),
+                ),
+                "fdm run (resident)",
+            )
+            return
         if codegen.is_walk(tile) or codegen.is_march(tile) or stage:
             # these kernels move up to 16 bytes per access: every buffer,
             # instance and step must start on a 16-byte boundary
@@ -888,6 +904,22 @@ class StencilPlan:
             ),
             "fdm run",
         )
+
+    def _stages(self) -> int:
+        gen = self.module.gen
+        return codegen.stage_count(gen.integrator, gen.invariant, 0)
+
+    def resident_shape(self) -> Optional[Tuple[int, int]]:
+        """(CTAs per instance, rows per CTA) of the resident kernel, or None
+        (``codegen.resident_shape``)."""
+        if self._resident is False:
+            cluster = ctypes.c_int()
+            tile = codegen.RESIDENT_TILE
+            if self.rows * self.ny <= codegen.RESIDENT_VERTICES[self.esize]:
+                _native.check(_native.lib().prml_kernel_max_cluster(self._step_kernel(tile), tile[2],
+                                                                    ctypes.byref(cluster)), "cluster size")
+            self._resident = codegen.resident_shape(self.rows, self.ny, self.C, self.esize, self._stages(), cluster.value)
+        return self._resident
 
     def march_rows(self, tile, batch: int) -> Tuple[int, int]:
         """Rows per job of a marching kernel for ``batch`` instances
@@ -977,6 +1009,8 @@ class StencilPlan:
 
         sms = _torch.cuda.get_device_properties(self.device).multi_processor_count
         cands = list(self.module.gen.step_kernels) + list(getattr(self.module.gen, "march_kernels", {}))
+        if getattr(self.module.gen, "resident_kernels", {}) and self.resident_shape() is not None:
+            cands += list(self.module.gen.resident_kernels)
         stage = list(getattr(self.module.gen, "stage_kernels", {}))
         if stage and 3 * self.batch * self.inst * self.esize <= STAGE_WORK_BYTES:
             cands += stage
@@ -1000,7 +1034,8 @@ class StencilPlan:
                 # fewer CTAs per SM that each walk several tiles and stage the
                 # next tile while computing the current one
                 # (marching jobs are sized by their rows instead)
-                caps = [0] + [sms * c for c in (2, 4, 8) if c < occ.value and not (codegen.is_march(tile) or codegen.is_stage(tile))]
+                caps = [0] + [sms * c for c in (2, 4, 8) if c < occ.value 
+                              and not (codegen.is_march(tile) or codegen.is_stage(tile) or codegen.is_resident(tile))]
 
                 def go(n, tile=tile):
                     self._launch(
@@ -1029,6 +1064,8 @@ class StencilPlan:
                 self.params.max_ctas = cap
                 rounds = max(1, min(16, int(2.0 / max(ms1, 1e-3))))
                 ms = min(timed(rounds) for _ in range(3)) / rounds
+                if codegen.is_resident(tile):  # must win clearly: fewer instances do not make it faster
+                    ms *= 1.05
                 if ms < best_t:
                     best, best_caps, best_t = tile, cap, ms
         finally:
