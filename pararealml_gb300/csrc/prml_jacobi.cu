@@ -847,6 +847,11 @@ bool staged_shape(const prml_jacobi_params& p, int sms, Stage<T>& sg, int& G, in
 constexpr int CT = 512;  // threads per CTA
 constexpr int CK = 16;   // iterations between two stop tests
 constexpr int CL_MAX = 16;
+/* The sums of consecutive blocks go to alternating copies: a CTA may send the
+ * next block's before another has read this block's (a last block of few
+ * iterations is over before the wait for a halo reaches that CTA); the cluster
+ * barrier of the block between orders the reuse of a copy. */
+constexpr int SUM_COPIES = 2;
 
 __device__ __forceinline__ unsigned cluster_rank() {
   unsigned r;
@@ -898,7 +903,7 @@ __global__ void __launch_bounds__(CT) jacobi_cluster(const prml_jacobi_params p,
                                                      const double* __restrict__ y_init, unsigned char* scratch,
                                                      Layout L, Div d12, Div d2, Split sp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double cpart[CK][CL_MAX]; /* [iteration][CTA] squared changes of the block */
+  __shared__ double cpart[SUM_COPIES][CK][CL_MAX]; /* [block's parity][iteration][CTA] squared changes */
   __shared__ unsigned long long bar[2]; /* halo of copy 0 / 1 has arrived */
   __shared__ int hit_s, dead;
   const int n_lap = p.n_lap;
@@ -1080,7 +1085,7 @@ __global__ void __launch_bounds__(CT) jacobi_cluster(const prml_jacobi_params p,
 
   cluster_sync(); /* every CTA of the cluster runs, its barriers set, before its memory is written */
   publish(0);
-  int w = 0;
+  int w = 0, cp = 0; /* cp: the block's copy of the sums */
   long long it0 = 0;
   int result = -1; /* 0: no iteration, 1: stopped after it0, -1: not converged */
   if (!(__longlong_as_double(0x7ff0000000000000LL) > p.tol)) {
@@ -1108,7 +1113,7 @@ __global__ void __launch_bounds__(CT) jacobi_cluster(const prml_jacobi_params p,
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
           if (lane < sp.CL)
-            st_remote(remote_addr(&cpart[s][rank], lane), dead ? __longlong_as_double(0x7ff8000000000000LL) : double(a));
+            st_remote(remote_addr(&cpart[cp][s][rank], lane), dead ? __longlong_as_double(0x7ff8000000000000LL) : double(a));
         }
       }
       cluster_sync();
@@ -1116,14 +1121,15 @@ __global__ void __launch_bounds__(CT) jacobi_cluster(const prml_jacobi_params p,
         bool stop = false;
         if ((int)threadIdx.x < Kb) {
           double t = 0.0;
-          for (int r = 0; r < sp.CL; ++r) t += cpart[threadIdx.x][r];
+          for (int r = 0; r < sp.CL; ++r) t += cpart[cp][threadIdx.x][r];
           stop = !(sqrt(t) > p.tol);
         }
         const unsigned m = __ballot_sync(0xffffffffu, stop);
         if (threadIdx.x == 0) hit_s = m ? __ffs(m) - 1 : -1;
       }
       __syncthreads();
-      const int hit = hit_s; /* the same in every CTA; cpart is next written after a cluster barrier */
+      const int hit = hit_s; /* the same in every CTA */
+      cp ^= 1;
       if (hit >= 0) {
         it0 += hit + 1;
         result = 1;
