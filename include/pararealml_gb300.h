@@ -75,14 +75,16 @@ int prml_kernel_max_cluster(void* kernel, int block, int* cluster);
 /* prml_fdm_run for a resident kernel: all steps in one launch (at most 16384
  * steps, or save_every, per launch), a cluster of `cluster` CTAs per instance
  * with `band` rows each and `buffers` states in shared memory (2; steps of
- * several stages 4). */
+ * several stages 4).  base->max_ctas (at least `cluster`): as many instances
+ * per launch as it leaves room for. */
 int prml_resident_params_size(void);
 int prml_fdm_run_resident(void* kernel, int block, int cluster, int band, int comps, int buffers,
                           const prml_step_params* base, const void* y0, long long y0_bstride, void* traj,
                           long long traj_bstride, long long traj_step_stride, long long n_steps, int save_every, double t0,
                           double dt, void* stream);
 /* prml_fdm_run for a stage kernel of a 3D module: one launch per integrator
- * stage, each thread one 16-byte vector on `planes` planes.  stage_a and acc
+ * stage (more where base->max_ctas is below a stage's CTAs), each thread one
+ * 16-byte vector on `planes` planes.  stage_a and acc
  * (more than one stage), stage_b (more than two): work states with instances
  * work_bstride elements apart. */
 int prml_stage_params_size(void);

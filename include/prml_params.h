@@ -48,7 +48,10 @@ typedef struct prml_step_params {
   double inv_dxx0, inv_dxx1; /* 1 / (dx * dx)                           */
   double two_dx0, two_dx1;   /* 2 dx (Neumann ghost offset)             */
   int in_slot;             /* slot coordinate of `in` in its tensor map */
-  int max_ctas;            /* cap on the persistent grid, 0 = fill the GPU */
+  int max_ctas;            /* most CTAs of a launch, 0 = fill the GPU; step
+                              kernels whose work takes more run in several
+                              launches (stage kernels: block0; resident
+                              kernels: whole instances)                  */
   int* status;             /* device flag set to 1 when a bounded wait
                               inside a kernel times out (may be NULL)    */
   /* temporal blocking: a kernel built for tb_max > 1 takes tb_steps time
@@ -154,7 +157,7 @@ typedef struct prml_stage_params {
   void* acc;             /* slope sums; planes of LHS.Y rows hold their value */
   long long acc_bstride;
   int stage;
-  int pad;
+  int block0;            /* first of the stage's blocks that this launch takes */
 } prml_stage_params;
 
 /* ---- all steps of a small mesh in one launch ------------------------------

@@ -515,8 +515,9 @@ __device__ __forceinline__ void stage_body3(const prml_step_params& p, const prm
   const unsigned vecs = (unsigned)(p.ny + VW - 1) / VW;
   const unsigned jobs = (unsigned)((p.nz + Z - 1) / Z) * (unsigned)p.nx * vecs;
   const unsigned blocks = (jobs + NT - 1) / NT;
-  const unsigned b = blockIdx.x / blocks;
-  unsigned job = (blockIdx.x - b * blocks) * NT + threadIdx.x;
+  const unsigned block = (unsigned)sp.block0 + blockIdx.x;
+  const unsigned b = block / blocks;
+  unsigned job = (block - b * blocks) * NT + threadIdx.x;
   const bool active = job < jobs;
   if (!active) job = jobs - 1; /* takes part in the shuffles, stores nothing */
   const unsigned line = job / vecs;

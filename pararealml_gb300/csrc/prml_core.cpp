@@ -622,6 +622,10 @@ int prml_fdm_run_resident(void* kernel, int block, int cluster, int band, int co
   const long long smem = (long long)buffers * comps * scomp * base->elem_bytes;
   if (smem > k->smem) return fail(PRML_ERR_ARG, "prml_fdm_run_resident: the bands do not fit in shared memory");
   rp.scomp = (int)scomp;
+  /* a grid cap: as many whole instances per launch as it leaves room for */
+  if (base->max_ctas > 0 && base->max_ctas < cluster)
+    return fail(PRML_ERR_ARG, "prml_fdm_run_resident: an instance's cluster has more CTAs than max_ctas allows");
+  const int group = base->max_ctas > 0 && base->max_ctas / cluster < base->batch ? base->max_ctas / cluster : base->batch;
   if (cluster > 8)
     PRML_CU(g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1));
   prml_step_params p = *base;
@@ -635,18 +639,23 @@ int prml_fdm_run_resident(void* kernel, int block, int cluster, int band, int co
   long long cur_bstride = y0_bstride;
   for (long long done = 0; done < n_steps; done += chunk) {
     rp.n_steps = n_steps - done < chunk ? n_steps - done : chunk;
-    p.in = cur;
     p.in_bstride = cur_bstride;
     char* out = static_cast<char*>(traj) + (size_t)(done / save_every) * traj_step_stride * base->elem_bytes;
-    p.out = out;
     p.out_bstride = traj_bstride;
     p.t = t0 + (double)done * dt;
     p.bc_slot0 = base->bc_slot0 + (int)(2 * done);
-    CUlaunchConfig cfg;
-    CUlaunchAttribute attr;
-    cluster_config(&cfg, &attr, cluster, (long long)cluster * base->batch, block, (int)smem, static_cast<CUstream>(stream));
-    void* args[] = {&p, &rp};
-    PRML_CU(g_drv.LaunchKernelEx(&cfg, k->fn, args, nullptr));
+    for (int b = 0; b < base->batch; b += group) {
+      p.batch = base->batch - b < group ? base->batch - b : group;
+      p.in = cur + (size_t)b * cur_bstride * base->elem_bytes;
+      p.out = out + (size_t)b * traj_bstride * base->elem_bytes;
+      p.t_offset = base->t_offset ? base->t_offset + b : nullptr;
+      p.bc_inst_slot = base->bc_inst_slot ? base->bc_inst_slot + b : nullptr;
+      CUlaunchConfig cfg;
+      CUlaunchAttribute attr;
+      cluster_config(&cfg, &attr, cluster, (long long)cluster * p.batch, block, (int)smem, static_cast<CUstream>(stream));
+      void* args[] = {&p, &rp};
+      PRML_CU(g_drv.LaunchKernelEx(&cfg, k->fn, args, nullptr));
+    }
     cur = out + (size_t)(rp.n_steps / save_every - 1) * traj_step_stride * base->elem_bytes;
     cur_bstride = traj_bstride;
   }
@@ -679,7 +688,8 @@ int prml_fdm_run_stages(void* kernel, int block, int planes, const prml_step_par
   const long long blocks = (jobs + block - 1) / block * base->batch;
   if (jobs + block >= (1LL << 31) || blocks >= (1LL << 31))
     return fail(PRML_ERR_ARG, "too many tiles for one launch (2^31)");
-  const int grid = (int)blocks;
+  /* a grid cap: the blocks of a stage in several launches */
+  const long long grid = base->max_ctas > 0 && base->max_ctas < blocks ? base->max_ctas : blocks;
   const size_t ebytes = (size_t)base->elem_bytes;
   prml_step_params p = *base;
   p.tb_steps = 1;
@@ -714,8 +724,12 @@ int prml_fdm_run_stages(void* kernel, int block, int planes, const prml_step_par
       p.in_bstride = s == 0 ? cur_bstride : work_bstride;
       p.out = last ? out : static_cast<char*>((s & 1) ? stage_b : stage_a);
       p.out_bstride = last ? out_bstride : work_bstride;
-      rc = launch_step(k, block, grid, &p, &sp, static_cast<CUstream>(stream));
-      if (rc) return rc;
+      for (long long block0 = 0; block0 < blocks; block0 += grid) {
+        sp.block0 = (int)block0;
+        rc = launch_step(k, block, (int)(blocks - block0 < grid ? blocks - block0 : grid), &p, &sp,
+                         static_cast<CUstream>(stream));
+        if (rc) return rc;
+      }
     }
     cur = out;
     cur_bstride = out_bstride;

@@ -302,10 +302,13 @@ class StencilPlan:
         )
 
     def limit_ctas(self, max_ctas: int) -> None:
-        """Caps the persistent grid (0 = as many CTAs as fit on the GPU, or
+        """Caps the CTAs of a launch (0 = as many CTAs as fit on the GPU, or
         the cap the autotuner found best for the problem)."""
         self._user_ctas = int(max_ctas)
         self.params.max_ctas = int(max_ctas)
+        self._resident = False  # a cluster of at most max_ctas CTAs
+        self._tuned.clear()  # tuned among other kernels (autotune)
+        self._tuned_ctas.clear()
 
     def set_t_offset(self, t_offset) -> None:
         """Per-instance time offsets (device float64 tensor of length batch) or None."""
@@ -853,7 +856,7 @@ class StencilPlan:
         if codegen.is_resident(tile):
             shape = self.resident_shape()
             if shape is None:
-                raise ValueError("the mesh is too large for the resident step kernel")
+                raise ValueError("the mesh is too large, or max_ctas too small, for the resident step kernel")
             cluster, band = shape
             self.params.jobs_per_cta = 1
             _native.check(
@@ -918,7 +921,8 @@ class StencilPlan:
             if self.rows * self.ny <= codegen.RESIDENT_VERTICES[self.esize]:
                 _native.check(_native.lib().prml_kernel_max_cluster(self._step_kernel(tile), tile[2],
                                                                     ctypes.byref(cluster)), "cluster size")
-            self._resident = codegen.resident_shape(self.rows, self.ny, self.C, self.esize, self._stages(), cluster.value)
+            most = min(cluster.value, self._user_ctas) if self._user_ctas else cluster.value
+            self._resident = codegen.resident_shape(self.rows, self.ny, self.C, self.esize, self._stages(), most)
         return self._resident
 
     def march_rows(self, tile, batch: int) -> Tuple[int, int]:
@@ -986,6 +990,26 @@ class StencilPlan:
         self.params.bc_stride = int(np.prod(low.dirichlet.shape))
         self._dyn_key = key
 
+    def _capped(self) -> bool:
+        """Whether a caller's grid cap narrows the autotuner's choice."""
+        gen = self.module.gen
+        return bool((getattr(gen, "resident_kernels", {}) or getattr(gen, "stage_kernels", {})) and self._user_ctas)
+
+    def _candidates(self) -> list:
+        """Tiles of the kernels that the autotuner may choose from.  With a
+        caller's grid cap only the kernels whose CTAs walk over their tiles:
+        the others would take a launch per ``max_ctas`` CTAs."""
+        gen = self.module.gen
+        cands = list(gen.step_kernels) + list(getattr(gen, "march_kernels", {}))
+        resident, stage = getattr(gen, "resident_kernels", {}), getattr(gen, "stage_kernels", {})
+        if self._capped():
+            return cands
+        if resident and self.resident_shape() is not None:
+            cands += list(resident)
+        if stage and 3 * self.batch * self.inst * self.esize <= STAGE_WORK_BYTES:
+            cands += list(stage)
+        return cands
+
     def autotune(self, dt: float, full: bool = True) -> Tuple[int, ...]:
         """Times every instantiated tile on this problem and keeps the fastest.
 
@@ -1000,6 +1024,8 @@ class StencilPlan:
         if full in self._tuned:
             return self._tuned[full]
         key = f"{self.module.gen.key}:{self.nz}x{self.rows}x{self.ny}:b{self.batch}:{'full' if full else 'final'}:v3"
+        if self._capped():
+            key += ":capped"
         cached = _tune_cache_load().get(key)
         if isinstance(cached, dict) and tuple(cached.get("tile", ())) in self.module.gen.kernels:
             self._tuned[full] = tuple(cached["tile"])
@@ -1008,12 +1034,7 @@ class StencilPlan:
         import torch as _torch
 
         sms = _torch.cuda.get_device_properties(self.device).multi_processor_count
-        cands = list(self.module.gen.step_kernels) + list(getattr(self.module.gen, "march_kernels", {}))
-        if getattr(self.module.gen, "resident_kernels", {}) and self.resident_shape() is not None:
-            cands += list(self.module.gen.resident_kernels)
-        stage = list(getattr(self.module.gen, "stage_kernels", {}))
-        if stage and 3 * self.batch * self.inst * self.esize <= STAGE_WORK_BYTES:
-            cands += stage
+        cands = self._candidates()
         reps = 16  # a multiple of every temporal block; best of 3 rounds per tile
         # timing launches read boundary table 0 only: a time-dependent run's
         # tables may cover fewer half steps than the timing launches take
