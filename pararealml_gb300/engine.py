@@ -252,6 +252,8 @@ class StencilPlan:
         self.tile = tuple(tile) if tile is not None else None  # forced by the caller
         self._tuned: Dict[bool, Tuple[int, ...]] = {}  # trajectory pattern -> tuned tile
         self._tuned_ctas: Dict[bool, int] = {}  # trajectory pattern -> tuned grid cap (0 = fill the GPU)
+        # trajectory pattern -> fastest whole-step tile and its grid cap, where the tuned one is a stage kernel
+        self._tuned_whole: Dict[bool, Tuple[Tuple[int, ...], int]] = {}
         self._user_ctas = 0
         self._march_rows: Dict[tuple, Tuple[int, int]] = {}
         self._resident = False  # resident_shape(), once asked for
@@ -719,6 +721,8 @@ class StencilPlan:
         ``bc_inst_slot_ptr`` (device int32 per instance, in half steps) lets
         the instances of one launch start at different times of it.
         """
+        import torch
+
         if n_steps == 0:
             return
         # per-run records: one entry per step (implicit integrators, Jacobi
@@ -782,14 +786,24 @@ class StencilPlan:
                     work, n_steps, save_every, t0, dt,
                 )
                 return
-            self._launch(
-                tile, _addr(y0), self.inst if y0_bstride is None else y0_bstride,
+            args = (
+                _addr(y0), self.inst if y0_bstride is None else y0_bstride,
                 _addr(traj), self.inst if traj_bstride is None else traj_bstride,
                 self.params.batch * self.inst if traj_step_stride is None else traj_step_stride,
                 _addr(work[0]) if work is not None else 0,
                 _addr(work[1]) if work is not None else 0,
                 n_steps, save_every, t0, dt,
             )
+            try:
+                self._launch(tile, *args)
+            except torch.cuda.OutOfMemoryError:
+                # no room for the stage kernels' work states (nothing has been
+                # launched yet): the tuned whole-step kernel needs none
+                if self.tile is not None or not codegen.is_stage(tile):
+                    raise
+                self.last_tile, ctas = self._tuned_whole[full]
+                self.params.max_ctas = self.last_ctas = self._user_ctas or ctas
+                self._launch(self.last_tile, *args)
         finally:
             self.params.batch, self.params.t_offset = saved
             self.params.dirichlet, self.params.neumann = saved_tables
@@ -1030,6 +1044,10 @@ class StencilPlan:
         if isinstance(cached, dict) and tuple(cached.get("tile", ())) in self.module.gen.kernels:
             self._tuned[full] = tuple(cached["tile"])
             self._tuned_ctas[full] = int(cached.get("ctas", 0))
+            if codegen.is_stage(self._tuned[full]):
+                whole = tuple(cached.get("whole", ()))
+                self._tuned_whole[full] = ((whole, int(cached["whole_ctas"])) if whole in self.module.gen.step_kernels
+                                           else (next(iter(self.module.gen.step_kernels)), 0))
             return self._tuned[full]
         import torch as _torch
 
@@ -1074,10 +1092,16 @@ class StencilPlan:
                     stop.synchronize()
                     return start.elapsed_time(stop)
 
-                for cap in caps:
-                    self.params.max_ctas = cap
-                    go(2)
-                    timings.append((min(timed(1) for _ in range(3)), tile, cap, timed))
+                try:
+                    for cap in caps:
+                        self.params.max_ctas = cap
+                        go(2)
+                        timings.append((min(timed(1) for _ in range(3)), tile, cap, timed))
+                except torch.cuda.OutOfMemoryError:
+                    # no room for the stage kernels' work states
+                    if not codegen.is_stage(tile):
+                        raise
+                    timings = [e for e in timings if e[1] != tile]
             # the three fastest again with timings of at least ~2 ms each, so
             # that launch jitter does not pick the tile of a fast kernel
             best, best_caps, best_t = cands[0], 0, float("inf")
@@ -1102,7 +1126,12 @@ class StencilPlan:
             self.params.max_ctas = saved_ctas
         self._tuned[full] = best
         self._tuned_ctas[full] = best_caps
-        _tune_cache_store(key, {"tile": list(best), "ctas": best_caps})
+        entry = {"tile": list(best), "ctas": best_caps}
+        if codegen.is_stage(best):
+            _, whole, ctas, _ = min((e for e in timings if not codegen.is_stage(e[1])), key=lambda e: e[0])
+            self._tuned_whole[full] = (whole, ctas)
+            entry.update(whole=list(whole), whole_ctas=ctas)
+        _tune_cache_store(key, entry)
         return best
 
 

@@ -67,7 +67,7 @@ def test_a_cap_leaves_the_walking_kernels_to_the_autotuner(monkeypatch, build, i
     monkeypatch.setattr(engine, "_tune_cache_load", lambda: stored)
     monkeypatch.setattr(engine, "_tune_cache_store", lambda key, entry: stored.update({key: entry}))
     plan = object.__new__(engine.StencilPlan)
-    plan.tile, plan._tuned, plan._tuned_ctas, plan._resident = None, {}, {}, (4, 4)
+    plan.tile, plan._tuned, plan._tuned_ctas, plan._tuned_whole, plan._resident = None, {}, {}, {}, (4, 4)
     plan.module = types.SimpleNamespace(gen=gen)
     plan.nz, plan.rows, plan.ny, plan.C, plan.esize, plan.batch, plan.inst = 1, 17, 17, 1, 8, 1, 1
     plan.device = "cuda"
