@@ -472,7 +472,9 @@ int prml_fdm_run(void* kernel, int block, int tile_x, int tile_y, int box_rows, 
                  int save_every, double t0, double dt, void* stream) {
   Kernel* k = static_cast<Kernel*>(kernel);
   if (!k) return fail(PRML_ERR_ARG, "prml_fdm_run: null kernel");
-  int rc = check_geometry(base, tile_x, tile_y, block);
+  /* a marching kernel's tile_x is no row count: its jobs are bounded below */
+  const bool march = base && base->jobs_per_cta > 1;
+  int rc = check_geometry(base, march ? (base->nx < 1 ? 1 : base->nx) : tile_x, tile_y, block);
   if (rc) return rc;
   if (!y0 || !traj || n_steps < 0 || save_every < 1 || comps < 1)
     return fail(PRML_ERR_ARG, "prml_fdm_run: bad buffers or step counts");
