@@ -1024,6 +1024,23 @@ class StencilPlan:
             cands += list(stage)
         return cands
 
+    # raised whenever the choice among the marching, stage and resident
+    # kernels changes, so that picks stored under the rule before are not taken
+    TUNE_RULE = 2
+
+    def _tune_key(self, full: bool) -> str:
+        """Cache key of a tuning.  Modules with marching, stage or resident
+        kernels: also the device, whose SMs and cluster size decide which of
+        them can run, and whether a grid cap leaves some of them out."""
+        import torch
+
+        gen = self.module.gen
+        key = f"{gen.key}:{self.nz}x{self.rows}x{self.ny}:b{self.batch}:{'full' if full else 'final'}:v3"
+        if any(getattr(gen, kind, {}) for kind in ("march_kernels", "stage_kernels", "resident_kernels")):
+            device = torch.cuda.get_device_properties(self.device)
+            key += f":{device.name}:{device.multi_processor_count}:r{self.TUNE_RULE}"
+        return key + ":capped" if self._capped() else key
+
     def autotune(self, dt: float, full: bool = True) -> Tuple[int, ...]:
         """Times every instantiated tile on this problem and keeps the fastest.
 
@@ -1037,11 +1054,10 @@ class StencilPlan:
             return self.tile
         if full in self._tuned:
             return self._tuned[full]
-        key = f"{self.module.gen.key}:{self.nz}x{self.rows}x{self.ny}:b{self.batch}:{'full' if full else 'final'}:v3"
-        if self._capped():
-            key += ":capped"
+        cands = self._candidates()
+        key = self._tune_key(full)
         cached = _tune_cache_load().get(key)
-        if isinstance(cached, dict) and tuple(cached.get("tile", ())) in self.module.gen.kernels:
+        if isinstance(cached, dict) and tuple(cached.get("tile", ())) in cands:
             self._tuned[full] = tuple(cached["tile"])
             self._tuned_ctas[full] = int(cached.get("ctas", 0))
             if codegen.is_stage(self._tuned[full]):
@@ -1052,7 +1068,6 @@ class StencilPlan:
         import torch as _torch
 
         sms = _torch.cuda.get_device_properties(self.device).multi_processor_count
-        cands = self._candidates()
         reps = 16  # a multiple of every temporal block; best of 3 rounds per tile
         # timing launches read boundary table 0 only: a time-dependent run's
         # tables may cover fewer half steps than the timing launches take

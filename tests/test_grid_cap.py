@@ -22,18 +22,10 @@ def _gen(ivp, integ, dtype="f64"):
     return codegen.generate_source(codegen.lower_problem(ivp.constrained_problem), integ, dtype, fast=True)
 
 
-@pytest.mark.parametrize("cap", [0, 3])
-@pytest.mark.parametrize("build,integ", [
-    (lambda: problems.diffusion_3d_mixed(ns), codegen.RK4),
-    (lambda: problems.diffusion_2d(ns, n=16), codegen.FORWARD_EULER),
-])
-def test_a_cap_leaves_the_walking_kernels_to_the_autotuner(monkeypatch, build, integ, cap):
-    """autotune() with the device calls replaced: stage and resident kernels
-    are the fastest, and are timed only without a cap."""
+def tuning_plan(monkeypatch, gen, cost, stored):
+    """A plan whose autotune() runs on a clock that ``cost(tile)`` advances
+    per launch, with ``stored`` as the cache; and the set of tiles it times."""
     torch = pytest.importorskip("torch")
-    gen = _gen(build(), integ)
-    special = {**gen.stage_kernels, **gen.resident_kernels}
-    assert special
     clock, timed = [0.0], set()
 
     class Event:
@@ -58,7 +50,6 @@ def test_a_cap_leaves_the_walking_kernels_to_the_autotuner(monkeypatch, build, i
         occ._obj.value = 1
         return 0
 
-    stored = {}
     monkeypatch.setattr(torch.cuda, "Event", Event)
     monkeypatch.setattr(torch.cuda, "get_device_properties",
                         lambda dev: types.SimpleNamespace(multi_processor_count=152, name="GPU"))
@@ -70,7 +61,7 @@ def test_a_cap_leaves_the_walking_kernels_to_the_autotuner(monkeypatch, build, i
     plan.tile, plan._tuned, plan._tuned_ctas, plan._tuned_whole, plan._resident = None, {}, {}, {}, (4, 4)
     plan.module = types.SimpleNamespace(gen=gen)
     plan.nz, plan.rows, plan.ny, plan.C, plan.esize, plan.batch, plan.inst = 1, 17, 17, 1, 8, 1, 1
-    plan.device = "cuda"
+    plan.device, plan._user_ctas = "cuda", 0
     plan.params = types.SimpleNamespace(bc_stride=0, max_ctas=0)
     plan.new_state = lambda n: State()
     plan._step_kernel = lambda tile: tile
@@ -78,9 +69,23 @@ def test_a_cap_leaves_the_walking_kernels_to_the_autotuner(monkeypatch, build, i
 
     def launch(tile, *a):
         timed.add(tile)
-        clock[0] += 0.1 if tile in special else 0.2
+        clock[0] += cost(tile)
 
     plan._launch = launch
+    return plan, timed
+
+
+@pytest.mark.parametrize("cap", [0, 3])
+@pytest.mark.parametrize("build,integ", [
+    (lambda: problems.diffusion_3d_mixed(ns), codegen.RK4),
+    (lambda: problems.diffusion_2d(ns, n=16), codegen.FORWARD_EULER),
+])
+def test_a_cap_leaves_the_walking_kernels_to_the_autotuner(monkeypatch, build, integ, cap):
+    """Stage and resident kernels are the fastest, and are timed only without a cap."""
+    gen = _gen(build(), integ)
+    special = {**gen.stage_kernels, **gen.resident_kernels}
+    assert special
+    plan, timed = tuning_plan(monkeypatch, gen, lambda tile: 0.1 if tile in special else 0.2, {})
     plan.limit_ctas(cap)
     best = plan.autotune(1e-4)
     assert (best in special) == (cap == 0) and bool(timed & set(special)) == (cap == 0)
