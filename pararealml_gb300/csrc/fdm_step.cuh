@@ -608,15 +608,39 @@ __device__ __forceinline__ int secant_tile(const prml_secant_params& s, int batc
   if (first && threadIdx.x == 0) *(volatile int*)(s.done + b) = prev;
   return SECANT_FINISH;
 }
-/* The counters of iteration k after a tile (every lane of the warp calls). */
-__device__ __forceinline__ void secant_count(const prml_secant_params& s, int batch, int b, bool changed, bool failing) {
-  if (s.iteration == 0) return;
-  int* cnt = s.counters + ((s.iteration % 3) * batch + b) * 2;
-  const bool ch = __any_sync(0xffffffffu, changed), fa = __any_sync(0xffffffffu, failing);
+/* What a CTA's tiles of one instance found so far.  Counters are written once
+ * per warp when the CTA goes on to another instance and once per CTA at the
+ * end, not per tile: every CTA's stores of an iteration meet in one cache line
+ * that all of them also read (secant_tile), and with a store per warp and tile
+ * an iteration of 513^2 took 352 us and of 1025^2 1543, 46 and 130 so (257^2: 18 either way). */
+struct SecantCount {
+  int b; /* instance, -1 before the first */
+  bool changed, failing;
+};
+/* counters of cnt.b (every lane of the warp calls) */
+__device__ __forceinline__ void secant_count(const prml_secant_params& s, int batch, const SecantCount& cnt) {
+  if (s.iteration == 0 || cnt.b < 0) return;
+  int* c = s.counters + ((s.iteration % 3) * batch + cnt.b) * 2;
+  const bool ch = __any_sync(0xffffffffu, cnt.changed), fa = __any_sync(0xffffffffu, cnt.failing);
   if ((threadIdx.x & 31) == 0) {
-    if (ch) cnt[0] = 1;
-    if (fa) cnt[1] = 1;
+    if (ch) c[0] = 1;
+    if (fa) c[1] = 1;
   }
+}
+/* before a tile of instance b */
+__device__ __forceinline__ void secant_enter(const prml_secant_params& s, int batch, int b, SecantCount& cnt) {
+  if (cnt.b == b) return;
+  secant_count(s, batch, cnt);
+  cnt = SecantCount{b, false, false};
+}
+/* after the last tile (every thread of the CTA calls) */
+__device__ __forceinline__ void secant_leave(const prml_secant_params& s, int batch, const SecantCount& cnt) {
+  if (s.iteration == 0 || cnt.b < 0) return;
+  const int ch = __syncthreads_or(cnt.changed), fa = __syncthreads_or(cnt.failing);
+  if (threadIdx.x != 0) return;
+  int* c = s.counters + ((s.iteration % 3) * batch + cnt.b) * 2;
+  if (ch) c[0] = 1;
+  if (fa) c[1] = 1;
 }
 
 /* Clears the counter set of the next iteration (block 0). */
@@ -822,13 +846,12 @@ __device__ __forceinline__ void secant_prefetch(const prml_step_params& p, const
 template <typename T, class Eq, int PER, int TX, int TY, int NT, bool EDGE>
 __device__ __forceinline__ void tile_secant(const prml_step_params& p, const MeshC<T>& m, const T* ybuf, int b, int gi0,
                                             int gj0, const prml_secant_params& s, int what, bool flat,
-                                            const SecantIn (&in)[PER][Eq::C]) {
+                                            const SecantIn (&in)[PER][Eq::C], SecantCount& cnt) {
   constexpr int C = Eq::C;
   constexpr int ND = Eq::ND;
   constexpr int HX = 1, HY = ColHalo<T, 1>::value;
   constexpr int RY = TY + 2 * HY, RXY = (TX + 2 * HX) * RY;
   const double t = Eq::USES_T ? p.t + (p.t_offset ? p.t_offset[b] : 0.0) : 0.0;
-  bool changed = false, failing = false;
   SecantTally tally{0, 0, 0.0};
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
@@ -855,11 +878,10 @@ __device__ __forceinline__ void tile_secant(const prml_step_params& p, const Mes
       for (int i = 0; i < ND; ++i)
         if (Eq::dcomp(i) == c) fc = f[i];
       const T target = dirichlet<T, Eq, EDGE>(secant_target(s, in[q][c], fc), c, gi, gj, m);
-      secant_element(s, e, in[q][c], x1, __dsub_rn(x1, target), changed, failing);
+      secant_element(s, e, in[q][c], x1, __dsub_rn(x1, target), cnt.changed, cnt.failing);
     }
   }
   if (what == SECANT_FINISH) secant_report(s.stats + 3 * b, tally);
-  else secant_count(s, p.batch, b, changed, failing);
 }
 
 /* Single-stage time steps on one staged tile, in one pass per step: the
@@ -1131,6 +1153,8 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
   Walk nxt = advance(cur);
   if (threadIdx.x == 0 && t < total) issue(cur, 0);
 
+  SecantCount sec_cnt{-1, false, false};
+  (void)sec_cnt;
   for (int it = 0; t < total; t += G, ++it) {
     const int buf = it & 1;
     const int next = t + G;
@@ -1162,9 +1186,12 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
     const bool edge = gi0 < HX + 1 || gi0 + TX + HX + 1 > p.nx || gj0 < HX + 1 || gj0 + TY + HX + 1 > p.ny;
     const T* ybuf = buf ? ybuf1 : ybuf0;
     if constexpr (MODE == 2) {
+      if (sec_what == SECANT_ITERATE) secant_enter(*sec, p.batch, b, sec_cnt);
       if (sec_what != SECANT_IDLE) {
-        if (edge) tile_secant<T, Eq, PER, TX, TY, NT, true>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in);
-        else tile_secant<T, Eq, PER, TX, TY, NT, false>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in);
+        if (edge)
+          tile_secant<T, Eq, PER, TX, TY, NT, true>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in, sec_cnt);
+        else
+          tile_secant<T, Eq, PER, TX, TY, NT, false>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in, sec_cnt);
       }
     } else if constexpr (MODE == 0 && NSTAGE == 1) {
       /* single-stage steps (one or TB per launch): one pass per step */
@@ -1178,6 +1205,7 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
     cur = nxt;
     nxt = advance(nxt);
   }
+  if constexpr (MODE == 2) secant_leave(*sec, p.batch, sec_cnt);
 }
 
 /* Mesh constants of a launch in the state type (float32 kernels read the

@@ -224,7 +224,7 @@ __device__ __forceinline__ void tma_load_5d3(void* dst, const TmaDesc* map, int 
 template <typename T, class Eq, int INTEG, int TZ, int TX, int TY, int NT, int MODE>
 __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const MeshC3<T>& m, const T* ybuf,
                                               T* bufA, T* bufB, int b, int gk0, int gi0, int gj0,
-                                              const prml_secant_params* sec = nullptr) {
+                                              const prml_secant_params* sec, SecantCount& sec_cnt) {
   constexpr int C = Eq::C;
   constexpr int ND = Eq::ND;
   constexpr int NSTAGE = (MODE != 0 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
@@ -243,11 +243,12 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
   T* nxt = bufA;
   (void)bufB;
   int sec_what = 0;
-  bool sec_changed = false, sec_failing = false, sec_flat = false;
+  bool sec_flat = false;
   SecantTally sec_tally{0, 0, 0.0};
   if constexpr (MODE == 2) {
     sec_what = secant_tile(*sec, p.batch, b, gk0 == 0 && gi0 == 0 && gj0 == 0, sec_flat);
     if (sec_what == SECANT_IDLE) return;
+    if (sec_what == SECANT_ITERATE) secant_enter(*sec, p.batch, b, sec_cnt);
   }
 
 #pragma unroll
@@ -288,7 +289,7 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
           for (int i = 0; i < ND; ++i)
             if (Eq::dcomp(i) == c) fc = f[i];
           const T target = dirichlet3<T, Eq>(secant_target(*sec, in, fc), c, g, ms);
-          secant_element(*sec, e, in, x1, __dsub_rn(x1, target), sec_changed, sec_failing);
+          secant_element(*sec, e, in, x1, __dsub_rn(x1, target), sec_cnt.changed, sec_cnt.failing);
         }
         return;
       }
@@ -359,7 +360,6 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
   }
   if constexpr (MODE == 2) {
     if (sec_what == SECANT_FINISH) secant_report(sec->stats + 3 * b, sec_tally);
-    else secant_count(*sec, p.batch, b, sec_changed, sec_failing);
   }
   if (MODE != 0) return;
 
@@ -459,6 +459,7 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
   __syncthreads();
   int t = blockIdx.x;
   if (threadIdx.x == 0 && t < total) issue(t, 0);
+  SecantCount sec_cnt{-1, false, false};
   for (int it = 0; t < total; t += gridDim.x, ++it) {
     const int buf = it & 1;
     const int next = t + gridDim.x;
@@ -474,9 +475,10 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
     int b, tz, ty, tx;
     coords(t, b, tz, ty, tx);
     tile_compute3<T, Eq, INTEG, TZ, TX, TY, NT, MODE>(p, m, buf ? ybuf1 : ybuf0, bufA, bufB, b, tz * TZ,
-                                                     ty * TX, tx * TY, sec);
+                                                     ty * TX, tx * TY, sec, sec_cnt);
     __syncthreads();
   }
+  if constexpr (MODE == 2) secant_leave(*sec, p.batch, sec_cnt);
 }
 
 /* One integrator stage per launch (prml_stage_params): a thread holds 16 bytes
