@@ -252,7 +252,8 @@ class StencilPlan:
         self.tile = tuple(tile) if tile is not None else None  # forced by the caller
         self._tuned: Dict[bool, Tuple[int, ...]] = {}  # trajectory pattern -> tuned tile
         self._tuned_ctas: Dict[bool, int] = {}  # trajectory pattern -> tuned grid cap (0 = fill the GPU)
-        # trajectory pattern -> fastest whole-step tile and its grid cap, where the tuned one is a stage kernel
+        # trajectory pattern -> fastest other tile and its grid cap, where the
+        # tuned one is a marching, stage or resident kernel
         self._tuned_whole: Dict[bool, Tuple[Tuple[int, ...], int]] = {}
         self._user_ctas = 0
         self._march_rows: Dict[tuple, Tuple[int, int]] = {}
@@ -1041,6 +1042,19 @@ class StencilPlan:
             key += f":{device.name}:{device.multi_processor_count}:r{self.TUNE_RULE}"
         return key + ":capped" if self._capped() else key
 
+    def tuned_choices(self, full: bool) -> list:
+        """(tile, grid cap) as tuned for this trajectory pattern and, where
+        that is a marching, stage or resident kernel, the fastest of the
+        other kernels."""
+        choices = [(self._tuned[full], self._tuned_ctas[full])]
+        if self._tuned[full] not in self.module.gen.step_kernels:
+            choices.append(self._tuned_whole[full])
+        return choices
+
+    def set_tuned(self, full: bool, choice) -> None:
+        """Runs of this trajectory pattern take ``choice`` (tile, grid cap) from now on."""
+        self._tuned[full], self._tuned_ctas[full] = choice
+
     def autotune(self, dt: float, full: bool = True) -> Tuple[int, ...]:
         """Times every instantiated tile on this problem and keeps the fastest.
 
@@ -1060,7 +1074,7 @@ class StencilPlan:
         if isinstance(cached, dict) and tuple(cached.get("tile", ())) in cands:
             self._tuned[full] = tuple(cached["tile"])
             self._tuned_ctas[full] = int(cached.get("ctas", 0))
-            if codegen.is_stage(self._tuned[full]):
+            if self._tuned[full] not in self.module.gen.step_kernels:
                 whole = tuple(cached.get("whole", ()))
                 self._tuned_whole[full] = ((whole, int(cached["whole_ctas"])) if whole in self.module.gen.step_kernels
                                            else (next(iter(self.module.gen.step_kernels)), 0))
@@ -1142,8 +1156,8 @@ class StencilPlan:
         self._tuned[full] = best
         self._tuned_ctas[full] = best_caps
         entry = {"tile": list(best), "ctas": best_caps}
-        if codegen.is_stage(best):
-            _, whole, ctas, _ = min((e for e in timings if not codegen.is_stage(e[1])), key=lambda e: e[0])
+        if best not in self.module.gen.step_kernels:
+            _, whole, ctas, _ = min((e for e in timings if e[1] in self.module.gen.step_kernels), key=lambda e: e[0])
             self._tuned_whole[full] = (whole, ctas)
             entry.update(whole=list(whole), whole_ctas=ctas)
         _tune_cache_store(key, entry)

