@@ -1010,21 +1010,19 @@ class StencilPlan:
         gen = self.module.gen
         return bool((getattr(gen, "resident_kernels", {}) or getattr(gen, "stage_kernels", {})) and self._user_ctas)
 
-    def _candidates(self) -> list:
-        """Tiles of the kernels that the autotuner may choose from.  With a
+    def _offers(self, tile) -> bool:
+        """Whether the autotuner may choose a tile of the module.  With a
         caller's grid cap only the kernels whose CTAs walk over their tiles:
         the others would take a launch per ``max_ctas`` CTAs."""
-        gen = self.module.gen
-        cands = list(gen.step_kernels) + list(getattr(gen, "march_kernels", {}))
-        resident, stage = getattr(gen, "resident_kernels", {}), getattr(gen, "stage_kernels", {})
-        if self._capped():
-            return cands
-        if resident and self.resident_shape() is not None:
-            cands += list(resident)
-        if stage and 3 * self.batch * self.inst * self.esize <= STAGE_WORK_BYTES:
-            cands += list(stage)
-        return cands
+        if codegen.is_stage(tile):
+            return not self._capped() and 3 * self.batch * self.inst * self.esize <= STAGE_WORK_BYTES
+        return not codegen.is_resident(tile) or (not self._capped() and self.resident_shape() is not None)
 
+    def _candidates(self) -> list:
+        """Tiles of the kernels that the autotuner may choose from."""
+        return [tile for kind in self.TUNED_KERNELS for tile in getattr(self.module.gen, kind, {}) if self._offers(tile)]
+
+    TUNED_KERNELS = ("step_kernels", "march_kernels", "resident_kernels", "stage_kernels")
     # raised whenever the choice among the marching, stage and resident
     # kernels changes, so that picks stored under the rule before are not taken
     TUNE_RULE = 2
@@ -1068,11 +1066,11 @@ class StencilPlan:
             return self.tile
         if full in self._tuned:
             return self._tuned[full]
-        cands = self._candidates()
         key = self._tune_key(full)
         cached = _tune_cache_load().get(key)
-        if isinstance(cached, dict) and tuple(cached.get("tile", ())) in cands:
-            self._tuned[full] = tuple(cached["tile"])
+        tile = tuple(cached.get("tile", ())) if isinstance(cached, dict) else ()
+        if any(tile in getattr(self.module.gen, kind, {}) for kind in self.TUNED_KERNELS) and self._offers(tile):
+            self._tuned[full] = tile
             self._tuned_ctas[full] = int(cached.get("ctas", 0))
             if self._tuned[full] not in self.module.gen.step_kernels:
                 whole = tuple(cached.get("whole", ()))
@@ -1082,6 +1080,7 @@ class StencilPlan:
         import torch as _torch
 
         sms = _torch.cuda.get_device_properties(self.device).multi_processor_count
+        cands = self._candidates()
         reps = 16  # a multiple of every temporal block; best of 3 rounds per tile
         # timing launches read boundary table 0 only: a time-dependent run's
         # tables may cover fewer half steps than the timing launches take
