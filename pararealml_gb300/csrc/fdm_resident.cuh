@@ -2,7 +2,7 @@
  * Every step of a small 2D mesh in one launch: one thread-block cluster per
  * instance holds the state in shared memory, each CTA a band of rows.
  *
- * Why: a launch per step costs 2.6 us on GB300 however small the mesh (the
+ * Why: a launch per step costs 2.4 us on GB300 however small the mesh (the
  * chain of dependent launches and a round trip through L2), which is all of a
  * 65^2 step.  Here a stage is: the warps with the band's two boundary rows
  * wait for the neighbour CTAs' rows (st.async into this CTA's halo rows,

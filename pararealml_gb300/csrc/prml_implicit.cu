@@ -18,14 +18,16 @@
  * (all elements to the midpoint), or after max_iterations steps.
  *
  * The kernels here are the element-wise parts (float64, rounded like the
- * numpy expressions: no contraction, IEEE division); the right-hand sides
- * come from the generated stencil module (prml_fdm_rhs).  Each instance
- * stops on its own counters, as separate reference solves would: the stop
- * test, the result copy and the status sums run on the device
- * (prml_implicit_stop, which also counts the iterations in device memory),
- * so the host can issue several iterations (or replay them as a CUDA graph)
- * before it reads whether every instance has finished; iterations of
- * finished instances leave them unchanged.
+ * numpy expressions: no contraction, IEEE division).  The package's own steps
+ * (prml_secant_solve) use predict, secant_stop and finish; their iterations
+ * are one launch each of the generated secant kernel (step_body's MODE 2),
+ * which also takes the stop test.  residual, update, status and stop are the
+ * same iteration in pieces for a caller of the C ABI who evaluates the
+ * right-hand sides with prml_fdm_rhs: the stop test, the result copy and the
+ * status sums run on the device (prml_implicit_stop, which also counts the
+ * iterations in device memory), so that several iterations can be issued (or
+ * replayed as a CUDA graph) before the host reads whether every instance has
+ * finished; iterations of finished instances leave them unchanged.
  */
 #include <cuda_runtime.h>
 

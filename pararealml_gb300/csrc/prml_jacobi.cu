@@ -839,7 +839,7 @@ bool staged_shape(const prml_jacobi_params& p, int sms, Stage<T>& sg, int& G, in
  * Why: the staged kernel pays a grid barrier through L2 per block and
  * recomputes its band's halo rows (7 rows for 4 owned at 101 x 81 in float64,
  * where the float64 pipe issues two operations per clock and SM).  At 101 x 81
- * an iteration takes 1.35 us in float64 (6.4 us staged) and 0.49 us in float32
+ * an iteration takes 1.33 us in float64 (6.6 us staged) and 0.47 us in float32
  * (2.8 us).  What is left in float64 is the pipe: 512 vertices x 6 operations
  * per SM are 0.8 us; in float32 the halo store, the neighbour's wait and the CTA
  * barrier.  A cluster barrier per iteration instead of the halo mbarriers took
@@ -1250,7 +1250,14 @@ int launch(const prml_jacobi_params& p, void* state, const double* y_init, void*
   Div d12 = make_div(p.n[1] * p.n[2]), d2 = make_div(p.n[2]);
   T* st = static_cast<T*>(state);
   unsigned char* sc = static_cast<unsigned char*>(scratch);
-  /* one cluster per instance where it fits */
+  /* one cluster per instance where it fits, whatever the batch: about nine
+   * clusters run at a time and the others follow, and the whole batch is still
+   * faster than on the staged kernel, which shares the GPU.  us per iteration
+   * of all instances in float64, staged against this: 101 x 81 with 1, 8, 16,
+   * 40 and 64 instances 6.6 / 1.33, 20.9 / 2.3, 33.9 / 3.5, 76 / 6.9, 119 / 11.4;
+   * 181 x 181 (the largest) with 1, 16 and 64 8.7 / 3.9, 44 / 11.6, 125 / 39;
+   * 31 x 32 x 33 with 1 and 32 32 / 5.4, 95 / 27; a 1D mesh of 400 with 1 and 64
+   * 4.5 / 0.69, 99 / 4.3; float32 gains more everywhere */
   Split sp{};
   int vt = 0;
   bool clustered = cluster_shape<T>(p, CL_MAX, sp, vt, smem);
