@@ -189,7 +189,7 @@ __device__ __forceinline__ void resident_body(const prml_step_params& p, const p
               res = yrhs[i];
             }
           }
-          res = dirichlet<T, Eq, true>(res, c, gi, j, me);
+          res = dirichlet<T, Eq, true, false>(res, c, gi, j, me);
           nxt[c * SC + l] = res;
           if (!end) {
             const unsigned off = shift + (unsigned)(c * SC + j) * (unsigned)sizeof(T);

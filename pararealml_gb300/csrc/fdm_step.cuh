@@ -58,11 +58,13 @@ __device__ __forceinline__ bool is_zero(double v) {
   return (((unsigned)__double2hiint(v) & 0x7fffffffu) | (unsigned)__double2loint(v)) == 0u;
 }
 
-/* The same test for `dirichlet`, as one integer comparison (a test of the two
- * halves in turn branches): RK4 steps of 1001 vertices in float64 3.8 -> 3.3
- * us, resident steps of 65^2 1.59 -> 1.41.  Not in the Neumann tests, the
- * marching and the 3D kernels, where it measured slower (24^3 RK4 stages 5 %,
- * 65^2 Cahn-Hilliard 6 %, 16 x 257^2 marching 0.8 %). */
+/* The same test as one integer comparison (a test of the two halves in turn
+ * branches), for the Dirichlet values of the staged and register-window
+ * kernels: RK4 steps in float64 of 1001 vertices 3.8 -> 3.3 us, of 161^2 9.6 ->
+ * 8.6.  Not where it measured slower: the Neumann tests (65^2 Cahn-Hilliard 6
+ * %), the marching kernels (16 x 257^2 0.8 %), the 3D kernels (24^3 RK4 stages
+ * 5 %) and the resident kernel, which takes 48 registers with it instead of 40
+ * (a single 65^2 instance 1.59 -> 1.41 us a step, but 16 of 41^2 1.6 -> 2.0). */
 __device__ __forceinline__ bool is_fixed(float v) { return v == v; }
 __device__ __forceinline__ bool is_fixed(double v) {
   return ((unsigned long long)__double_as_longlong(v) << 1) <= 0xffe0000000000000ull;
@@ -327,25 +329,26 @@ __device__ __forceinline__ constexpr bool has_dir(int f, int c) {
 }
 
 /* Dirichlet re-imposition with the reference's face precedence.  EDGE =
- * false: the vertex is known to be off every face (interior tile). */
-template <typename T, class Eq, bool EDGE = true>
+ * false: the vertex is known to be off every face (interior tile).  WHOLE:
+ * which test of an entry, see is_fixed. */
+template <typename T, class Eq, bool EDGE = true, bool WHOLE = true>
 __device__ __forceinline__ T dirichlet(T v, int c, int gi, int gj, const MeshC<T>& m) {
   if (!EDGE) return v;
   if (has_dir<Eq>(0, c) && gi == 0) {
     const T d = m.dir[(0 * Eq::C + c) * m.flen + gj];
-    if (is_fixed(d)) v = d;
+    if (WHOLE ? is_fixed(d) : is_value(d)) v = d;
   }
   if (has_dir<Eq>(1, c) && gi == m.nx - 1) {
     const T d = m.dir[(1 * Eq::C + c) * m.flen + gj];
-    if (is_fixed(d)) v = d;
+    if (WHOLE ? is_fixed(d) : is_value(d)) v = d;
   }
   if (has_dir<Eq>(2, c) && gj == 0) {
     const T d = m.dir[(2 * Eq::C + c) * m.flen + gi];
-    if (is_fixed(d)) v = d;
+    if (WHOLE ? is_fixed(d) : is_value(d)) v = d;
   }
   if (has_dir<Eq>(3, c) && gj == m.ny - 1) {
     const T d = m.dir[(3 * Eq::C + c) * m.flen + gi];
-    if (is_fixed(d)) v = d;
+    if (WHOLE ? is_fixed(d) : is_value(d)) v = d;
   }
   return v;
 }
