@@ -194,10 +194,10 @@ struct MarchPoint {
   }
 };
 
-/* What bounds it: instruction issue (float32: 125 warp instructions per row of
- * 64 columns for the four stages of RK4 diffusion, 72 % of the issue slots)
- * and the float64 pipe (80 % busy; 1.65 x the 23 operations per update that
- * diffusion needs, for the halo lanes and a chunk's first rows).  Measured, per 100
+/* What bounds it: instruction issue and latency (float32: 226 warp instructions
+ * per row of a strip for the four stages of RK4 diffusion with the face strips
+ * and a chunk's first rows counted in, 55 % of the issue slots while SMs are
+ * active) and the float64 pipe (82 % busy).  Measured, per 100
  * RK4 steps: 64 x 257^2 diffusion in float32 4.60 -> 2.43 ms, 16 x 257^2 in
  * float64 12.5 -> 9.1 ms (staged kernel before); 200 Cahn-Hilliard steps at
  * 1025^2 in float32 1.24 -> 0.95 ms with two steps per launch.  Three coupled

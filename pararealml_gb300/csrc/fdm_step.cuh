@@ -621,39 +621,26 @@ __device__ __forceinline__ int secant_tile(const prml_secant_params& s, int batc
   if (first && threadIdx.x == 0) *(volatile int*)(s.done + b) = prev;
   return SECANT_FINISH;
 }
-/* What a CTA's tiles of one instance found so far.  Counters are written once
- * per warp when the CTA goes on to another instance and once per CTA at the
- * end, not per tile: every CTA's stores of an iteration meet in one cache line
- * that all of them also read (secant_tile), and with a store per warp and tile
- * an iteration of 513^2 took 352 us and of 1025^2 1543, 46 and 130 so (257^2: 18 either way). */
-struct SecantCount {
-  int b; /* instance, -1 before the first */
-  bool changed, failing;
-};
-/* counters of cnt.b (every lane of the warp calls) */
-__device__ __forceinline__ void secant_count(const prml_secant_params& s, int batch, const SecantCount& cnt) {
-  if (s.iteration == 0 || cnt.b < 0) return;
-  int* c = s.counters + ((s.iteration % 3) * batch + cnt.b) * 2;
-  const bool ch = __any_sync(0xffffffffu, cnt.changed), fa = __any_sync(0xffffffffu, cnt.failing);
-  if ((threadIdx.x & 31) == 0) {
-    if (ch) c[0] = 1;
-    if (fa) c[1] = 1;
+/* What a warp found on a tile (every lane of the warp calls) joins what the
+ * CTA has found of the instance so far, in shared memory. */
+__device__ __forceinline__ void secant_count(const prml_secant_params& s, bool changed, bool failing, int* found) {
+  if (s.iteration == 0) return;
+  const int f = (__any_sync(0xffffffffu, changed) ? 1 : 0) | (__any_sync(0xffffffffu, failing) ? 2 : 0);
+  if ((threadIdx.x & 31) == 0 && (f & ~*(volatile int*)found)) atomicOr(found, f);
+}
+/* Thread 0, after the barrier that ends a tile of another instance (`last`; -1
+ * before the first) or the last tile: the counters of iteration k.  One store
+ * per CTA, not per warp and tile: the stores of all CTAs of an iteration meet in
+ * one cache line that all of them also read (secant_tile), and with a store per
+ * warp and tile an iteration of 513^2 took 352 us and of 1025^2 1543, 41 and 117
+ * so (257^2: 18 either way). */
+__device__ __forceinline__ void secant_tell(const prml_secant_params& s, int batch, int last, int* found) {
+  if (last >= 0) {
+    int* cnt = s.counters + ((s.iteration % 3) * batch + last) * 2;
+    if (*found & 1) cnt[0] = 1;
+    if (*found & 2) cnt[1] = 1;
   }
-}
-/* before a tile of instance b */
-__device__ __forceinline__ void secant_enter(const prml_secant_params& s, int batch, int b, SecantCount& cnt) {
-  if (cnt.b == b) return;
-  secant_count(s, batch, cnt);
-  cnt = SecantCount{b, false, false};
-}
-/* after the last tile (every thread of the CTA calls) */
-__device__ __forceinline__ void secant_leave(const prml_secant_params& s, int batch, const SecantCount& cnt) {
-  if (s.iteration == 0 || cnt.b < 0) return;
-  const int ch = __syncthreads_or(cnt.changed), fa = __syncthreads_or(cnt.failing);
-  if (threadIdx.x != 0) return;
-  int* c = s.counters + ((s.iteration % 3) * batch + cnt.b) * 2;
-  if (ch) c[0] = 1;
-  if (fa) c[1] = 1;
+  *found = 0;
 }
 
 /* Clears the counter set of the next iteration (block 0). */
@@ -859,12 +846,13 @@ __device__ __forceinline__ void secant_prefetch(const prml_step_params& p, const
 template <typename T, class Eq, int PER, int TX, int TY, int NT, bool EDGE>
 __device__ __forceinline__ void tile_secant(const prml_step_params& p, const MeshC<T>& m, const T* ybuf, int b, int gi0,
                                             int gj0, const prml_secant_params& s, int what, bool flat,
-                                            const SecantIn (&in)[PER][Eq::C], SecantCount& cnt) {
+                                            const SecantIn (&in)[PER][Eq::C], int* found) {
   constexpr int C = Eq::C;
   constexpr int ND = Eq::ND;
   constexpr int HX = 1, HY = ColHalo<T, 1>::value;
   constexpr int RY = TY + 2 * HY, RXY = (TX + 2 * HX) * RY;
   const double t = Eq::USES_T ? p.t + (p.t_offset ? p.t_offset[b] : 0.0) : 0.0;
+  bool changed = false, failing = false;
   SecantTally tally{0, 0, 0.0};
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
@@ -891,10 +879,11 @@ __device__ __forceinline__ void tile_secant(const prml_step_params& p, const Mes
       for (int i = 0; i < ND; ++i)
         if (Eq::dcomp(i) == c) fc = f[i];
       const T target = dirichlet<T, Eq, EDGE>(secant_target(s, in[q][c], fc), c, gi, gj, m);
-      secant_element(s, e, in[q][c], x1, __dsub_rn(x1, target), cnt.changed, cnt.failing);
+      secant_element(s, e, in[q][c], x1, __dsub_rn(x1, target), changed, failing);
     }
   }
   if (what == SECANT_FINISH) secant_report(s.stats + 3 * b, tally);
+  else secant_count(s, changed, failing, found);
 }
 
 /* Single-stage time steps on one staged tile, in one pass per step: the
@@ -1050,8 +1039,8 @@ __device__ __forceinline__ void tile_compute_tb(const prml_step_params& p, const
  * iteration of an implicit step (prml_secant_params; float64), one launch
  * where right-hand side, residual, update, stop test and result copy were
  * five.  us per iteration (whole steps over their iterations, backward Euler
- * diffusion), five launches against this: 257^2 40 / 18, 513^2 127 / 46, 1025^2
- * 531 / 130, 97^3 651 / 248.  The launch chain with its loads takes 6 us of it
+ * diffusion), five launches against this: 257^2 40 / 18, 513^2 127 / 41, 1025^2
+ * 531 / 117, 97^3 651 / 211.  The launch chain with its loads takes 6 us of it
  * (an idle iteration), the rest the float64 pipe: about 35 operations per
  * vertex, ten of them the secant's division. */
 template <typename T, class Eq, int INTEG, int TX, int TY, int NT, int MODE, int COMP = 0, int TB = 1>
@@ -1167,8 +1156,9 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
   Walk nxt = advance(cur);
   if (threadIdx.x == 0 && t < total) issue(cur, 0);
 
-  SecantCount sec_cnt{-1, false, false};
-  (void)sec_cnt;
+  __shared__ int sec_found;
+  int sec_last = -1;
+  (void)sec_last;
   for (int it = 0; t < total; t += G, ++it) {
     const int buf = it & 1;
     const int next = t + G;
@@ -1180,6 +1170,8 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
     int sec_what = 0;
     bool sec_flat = false;
     if constexpr (MODE == 2) {
+      if (threadIdx.x == 0 && cur.b != sec_last) secant_tell(*sec, p.batch, sec_last, &sec_found);
+      sec_last = cur.b;
       sec_what = secant_tile(*sec, p.batch, cur.b, cur.ty == 0 && cur.tx == 0, sec_flat);
       secant_prefetch<C, PER, TX, TY, NT>(p, *sec, cur.b, cur.ty * TX, cur.tx * TY, sec_in);
     }
@@ -1200,12 +1192,11 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
     const bool edge = gi0 < HX + 1 || gi0 + TX + HX + 1 > p.nx || gj0 < HX + 1 || gj0 + TY + HX + 1 > p.ny;
     const T* ybuf = buf ? ybuf1 : ybuf0;
     if constexpr (MODE == 2) {
-      if (sec_what == SECANT_ITERATE) secant_enter(*sec, p.batch, b, sec_cnt);
       if (sec_what != SECANT_IDLE) {
         if (edge)
-          tile_secant<T, Eq, PER, TX, TY, NT, true>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in, sec_cnt);
+          tile_secant<T, Eq, PER, TX, TY, NT, true>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in, &sec_found);
         else
-          tile_secant<T, Eq, PER, TX, TY, NT, false>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in, sec_cnt);
+          tile_secant<T, Eq, PER, TX, TY, NT, false>(p, m, ybuf, b, gi0, gj0, *sec, sec_what, sec_flat, sec_in, &sec_found);
       }
     } else if constexpr (MODE == 0 && NSTAGE == 1) {
       /* single-stage steps (one or TB per launch): one pass per step */
@@ -1219,7 +1210,9 @@ __device__ __forceinline__ void step_body(const prml_step_params& p, const TmaDe
     cur = nxt;
     nxt = advance(nxt);
   }
-  if constexpr (MODE == 2) secant_leave(*sec, p.batch, sec_cnt);
+  if constexpr (MODE == 2) {
+    if (threadIdx.x == 0) secant_tell(*sec, p.batch, sec_last, &sec_found);
+  }
 }
 
 /* Mesh constants of a launch in the state type (float32 kernels read the

@@ -224,7 +224,7 @@ __device__ __forceinline__ void tma_load_5d3(void* dst, const TmaDesc* map, int 
 template <typename T, class Eq, int INTEG, int TZ, int TX, int TY, int NT, int MODE>
 __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const MeshC3<T>& m, const T* ybuf,
                                               T* bufA, T* bufB, int b, int gk0, int gi0, int gj0,
-                                              const prml_secant_params* sec, SecantCount& sec_cnt) {
+                                              const prml_secant_params* sec, int* sec_found) {
   constexpr int C = Eq::C;
   constexpr int ND = Eq::ND;
   constexpr int NSTAGE = (MODE != 0 || Eq::STAGE_INVARIANT) ? 1 : INTEG;
@@ -243,12 +243,11 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
   T* nxt = bufA;
   (void)bufB;
   int sec_what = 0;
-  bool sec_flat = false;
+  bool sec_changed = false, sec_failing = false, sec_flat = false;
   SecantTally sec_tally{0, 0, 0.0};
   if constexpr (MODE == 2) {
     sec_what = secant_tile(*sec, p.batch, b, gk0 == 0 && gi0 == 0 && gj0 == 0, sec_flat);
     if (sec_what == SECANT_IDLE) return;
-    if (sec_what == SECANT_ITERATE) secant_enter(*sec, p.batch, b, sec_cnt);
   }
 
 #pragma unroll
@@ -289,7 +288,7 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
           for (int i = 0; i < ND; ++i)
             if (Eq::dcomp(i) == c) fc = f[i];
           const T target = dirichlet3<T, Eq>(secant_target(*sec, in, fc), c, g, ms);
-          secant_element(*sec, e, in, x1, __dsub_rn(x1, target), sec_cnt.changed, sec_cnt.failing);
+          secant_element(*sec, e, in, x1, __dsub_rn(x1, target), sec_changed, sec_failing);
         }
         return;
       }
@@ -360,6 +359,7 @@ __device__ __forceinline__ void tile_compute3(const prml_step_params& p, const M
   }
   if constexpr (MODE == 2) {
     if (sec_what == SECANT_FINISH) secant_report(sec->stats + 3 * b, sec_tally);
+    else secant_count(*sec, sec_changed, sec_failing, sec_found);
   }
   if (MODE != 0) return;
 
@@ -459,11 +459,18 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
   __syncthreads();
   int t = blockIdx.x;
   if (threadIdx.x == 0 && t < total) issue(t, 0);
-  SecantCount sec_cnt{-1, false, false};
+  __shared__ int sec_found;
+  int sec_last = -1;
+  (void)sec_last;
   for (int it = 0; t < total; t += gridDim.x, ++it) {
     const int buf = it & 1;
     const int next = t + gridDim.x;
     if (threadIdx.x == 0 && next < total) issue(next, buf ^ 1);
+    if constexpr (MODE == 2) {
+      const int b = t / per_inst;
+      if (threadIdx.x == 0 && b != sec_last) secant_tell(*sec, p.batch, sec_last, &sec_found);
+      sec_last = b;
+    }
     const unsigned long long wait_ns = p.wait_limit_ns ? p.wait_limit_ns : kWaitLimitNs;
     const bool ok = mbar_wait_bounded(&bar[buf], (unsigned)((it >> 1) & 1), wait_ns);
     if (__syncthreads_or(!ok)) {
@@ -475,10 +482,12 @@ __device__ __forceinline__ void step_body3(const prml_step_params& p, const TmaD
     int b, tz, ty, tx;
     coords(t, b, tz, ty, tx);
     tile_compute3<T, Eq, INTEG, TZ, TX, TY, NT, MODE>(p, m, buf ? ybuf1 : ybuf0, bufA, bufB, b, tz * TZ,
-                                                     ty * TX, tx * TY, sec, sec_cnt);
+                                                     ty * TX, tx * TY, sec, &sec_found);
     __syncthreads();
   }
-  if constexpr (MODE == 2) secant_leave(*sec, p.batch, sec_cnt);
+  if constexpr (MODE == 2) {
+    if (threadIdx.x == 0) secant_tell(*sec, p.batch, sec_last, &sec_found);
+  }
 }
 
 /* One integrator stage per launch (prml_stage_params): a thread holds 16 bytes
