@@ -40,3 +40,19 @@ def test_a_pick_of_another_device_or_rule_is_not_taken(monkeypatch, change):
     monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: device)
     plan.autotune(1e-4)
     assert timed
+
+
+def test_the_stored_picks_are_parsed_once_per_change(monkeypatch, tmp_path):
+    parses = []
+    load = engine.json.load
+    monkeypatch.setattr(engine.json, "load", lambda f: (parses.append(1), load(f))[1])
+    monkeypatch.setattr(engine._native, "JIT_CACHE_DIR", str(tmp_path))
+    assert engine._tune_cache_load() == {} and not parses
+    engine._tune_cache_store("a", {"tile": [1]})
+    for _ in range(3):
+        assert engine._tune_cache_load() == {"a": {"tile": [1]}}
+    assert len(parses) == 1
+    engine._tune_cache_store("b", {"tile": [2]})
+    assert engine._tune_cache_load() == {"a": {"tile": [1]}, "b": {"tile": [2]}} and len(parses) == 2
+    (tmp_path / "autotune.json").write_text("not json")
+    assert engine._tune_cache_load() == {}
