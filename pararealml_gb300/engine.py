@@ -733,8 +733,6 @@ class StencilPlan:
         ``bc_inst_slot_ptr`` (device int32 per instance, in half steps) lets
         the instances of one launch start at different times of it.
         """
-        import torch
-
         if n_steps == 0:
             return
         # per-run records: one entry per step (implicit integrators, Jacobi
@@ -808,10 +806,13 @@ class StencilPlan:
             )
             try:
                 self._launch(tile, *args)
-            except torch.cuda.OutOfMemoryError:
+            except RuntimeError as e:
+                import torch
+
                 # no room for the stage kernels' work states (nothing has been
                 # launched yet): the tuned whole-step kernel needs none
-                if self.tile is not None or not codegen.is_stage(tile):
+                if (not isinstance(e, torch.cuda.OutOfMemoryError) or self.tile is not None
+                        or not codegen.is_stage(tile)):
                     raise
                 self.last_tile, ctas = self._tuned_whole[full]
                 self.params.max_ctas = self.last_ctas = self._user_ctas or ctas
